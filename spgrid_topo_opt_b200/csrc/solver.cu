@@ -29,6 +29,7 @@
 
 #include "../../include/spgrid_fem.h"
 #include "band.hpp"
+#include "band_group.cuh"
 #include "common.cuh"
 #include "kernels.cuh"
 #include "setup.hpp"
@@ -84,6 +85,7 @@ struct Level {
   // then boundary sweep colours 8..15, concatenated; list k is gs_off[k]..gs_off[k+1]
   DevBuf<int> gs_list;
   int gs_off[17] = {0};
+  int gs_clear[16] = {0};  // where list k's entries that are only cleared begin
   // levels with stencils: node lists of the Gauss-Seidel passes, active nodes of
   // colour c (list c) and active boundary-band nodes of colour c (list 8 + c),
   // each ascending; list k is sgs_off[k]..sgs_off[k+1]
@@ -252,6 +254,16 @@ static double* cell_scratch(int slot, size_t count) {
   return c.p[slot];
 }
 
+// Tables of a level's boundary-band groups (band_group.cuh), shared by the
+// precisions of the level.
+struct BandTables {
+  BandPlan plan;
+  DevBuf<int> node;           // [BG_CTAS][slots] list entries
+  DevBuf<uint16_t> local;     // [BG_CTAS][slots][27] neighbours' local slots
+  DevBuf<uint16_t> push;      // [BG_CTAS][slots][BG_CTAS] halo slots an update goes to
+  DevBuf<int> hnode, hcount;  // [BG_CTAS][..] nodes of the halos, their numbers
+};
+
 class Solver {
  public:
   Problem P;
@@ -267,6 +279,7 @@ class Solver {
   // level data (double for reference/fp64, float for the mixed V-cycle)
   std::vector<std::unique_ptr<Level<double>>> L64;
   std::vector<std::unique_ptr<Level<float>>> L32;
+  std::vector<std::unique_ptr<BandTables>> band;  // per level; null where groups run pass by pass
   Bottom bottom;
   DevBuf<double> E64;
   DevBuf<float> E32;
@@ -342,6 +355,24 @@ class Solver {
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
+    SGS_CUDA(cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...));
+  }
+  // the same as one cluster of BG_CTAS CTAs
+  template <typename... KArgs, typename... Args>
+  void launch_group(void (*kernel)(KArgs...), size_t smem, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = BG_CTAS;
+    cfg.blockDim = BG_THREADS;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = BG_CTAS;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
     SGS_CUDA(cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...));
   }
   bool mixed() const { return precision == PREC_MIXED; }
@@ -540,15 +571,153 @@ class Solver {
     tmp.alloc(tmp_bytes);
     SGS_CUDA(cub::DeviceScan::ExclusiveSum(tmp.p, tmp_bytes, cnt.p, pos.p, int(n + 1), stream));
     // list k starts where sub-list 2k does (block 0); the end is the total
-    for (int k = 0; k < 16; ++k)
-      SGS_CUDA(cudaMemcpyAsync(&d.gs_off[k], pos.p + long(2 * k) * nb, sizeof(int), cudaMemcpyDeviceToHost, stream));
-    SGS_CUDA(cudaMemcpyAsync(&d.gs_off[16], pos.p + n, sizeof(int), cudaMemcpyDeviceToHost, stream));
+    int sub[33];
+    SGS_CUDA(cudaMemcpy2DAsync(sub, sizeof(int), pos.p, size_t(nb) * sizeof(int), sizeof(int), 32,
+                               cudaMemcpyDeviceToHost, stream));
+    SGS_CUDA(cudaMemcpyAsync(&sub[32], pos.p + n, sizeof(int), cudaMemcpyDeviceToHost, stream));
     SGS_CUDA(cudaStreamSynchronize(stream));
+    for (int k = 0; k < 16; ++k) {
+      d.gs_off[k] = sub[2 * k];
+      d.gs_clear[k] = sub[2 * k + 1];
+    }
+    d.gs_off[16] = sub[32];
     d.gs_list.alloc(size_t(d.gs_off[16]));
     if (d.gs_off[16] > 0)
       colour_fill_kernel<<<nb, 128, 0, stream>>>(nb, d.flags.p, band_block.p, pos.p, d.gs_list.p);
     SGS_CUDA(cudaGetLastError());
     SGS_CUDA(cudaStreamSynchronize(stream));  // the temporaries go out of scope
+  }
+
+  // Whether this device runs clusters of BG_CTAS CTAs of `kernel` with `smem`
+  // bytes of shared memory each.
+  template <typename K>
+  bool cluster_runs(K kernel, size_t smem) {
+    int most = 0;
+    SGS_CUDA(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
+    most -= 1024;  // the kernels' static shared memory
+    if (smem > size_t(std::max(0, most))) return false;
+    bool ok = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most) == cudaSuccess &&
+              cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+    if (ok) {
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = BG_CTAS;
+      cfg.blockDim = BG_THREADS;
+      cfg.dynamicSmemBytes = smem;
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = BG_CTAS;
+      attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      int n = 0;
+      ok = cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) == cudaSuccess && n > 0;
+    }
+    cudaGetLastError();
+    return ok;
+  }
+
+  // Tables of level l's boundary-band groups from its node lists 8..15, if a
+  // CTA's share of the band fits its shared memory in the V-cycle's precision.
+  // They depend on the hierarchy only: an operator update keeps them.
+  void band_tables(int l) {
+    band.resize(P.levels.size());
+    if (band[l] || P.boundary_smoothing <= 0) return;
+    Level<double>& d = *L64[l];
+    if (d.nbound == 0) return;
+    // the nodes a group updates, by colour (those that a level-0 pass only
+    // clears are zero throughout a V-cycle), from the lists on the device
+    const DevBuf<int>& list = l == 0 ? d.gs_list : d.sgs_list;
+    const int* lo = (l == 0 ? d.gs_off : d.sgs_off) + 8;
+    std::vector<int> entry(size_t(lo[8] - lo[0]));
+    if (entry.empty()) return;
+    SGS_CUDA(cudaMemcpyAsync(entry.data(), list.p + lo[0], entry.size() * sizeof(int), cudaMemcpyDeviceToHost, stream));
+    SGS_CUDA(cudaStreamSynchronize(stream));
+    std::vector<std::pair<int, int>> nodes;  // (node, colour), ascending
+    for (int c = 0; c < 8; ++c)
+      for (int k = lo[c]; k < (l == 0 ? d.gs_clear[8 + c] : lo[c + 1]); ++k) nodes.emplace_back(entry[size_t(k - lo[0])], c);
+    if (nodes.empty() || nodes.size() > 32768) return;
+    std::sort(nodes.begin(), nodes.end());
+    auto t = std::make_unique<BandTables>();
+    BandPlan& p = t->plan;
+    const size_t total = nodes.size();
+    auto owner = [&](size_t i) { return int(i * BG_CTAS / total); };
+    std::memset(p.own, 0, sizeof(p.own));
+    for (size_t i = 0; i < total; ++i) ++p.own[owner(i)][nodes[i].second];
+    for (int c = 0; c < 8; ++c) {
+      int most = 0;
+      for (int r = 0; r < BG_CTAS; ++r) most = std::max(most, int(p.own[r][c]));
+      p.off[c] = p.slots;
+      p.slots += most;
+    }
+    if (p.slots > BG_SLOTS) return;
+    std::vector<int> table(size_t(BG_CTAS) * p.slots, BG_NONE);
+    {
+      int at[BG_CTAS][8] = {};
+      for (size_t i = 0; i < total; ++i) {
+        const int r = owner(i), c = nodes[i].second;
+        table[size_t(r) * p.slots + size_t(p.off[c] + at[r][c]++)] = nodes[i].first;
+      }
+    }
+    DevBuf<uint32_t> map;
+    const int n = BG_CTAS * p.slots;
+    map.alloc(size_t(d.N));
+    t->node.alloc(size_t(n));
+    DevBuf<uint32_t> code;
+    code.alloc(size_t(n) * 27);
+    DevBuf<uint8_t> need;
+    need.alloc(size_t(n) * BG_CTAS);
+    need.zero(stream);
+    t->local.alloc(size_t(n) * 27);
+    t->push.alloc(size_t(n) * BG_CTAS);
+    t->hnode.alloc(size_t(n) * BG_CTAS);
+    t->hcount.alloc(BG_CTAS);
+    SGS_CUDA(cudaMemsetAsync(map.p, 0xff, size_t(d.N) * sizeof(uint32_t), stream));
+    SGS_CUDA(cudaMemcpyAsync(t->node.p, table.data(), size_t(n) * sizeof(int), cudaMemcpyHostToDevice, stream));
+    band_map_kernel<<<blocks_for(n, 256), 256, 0, stream>>>(n, p.slots, t->node.p, map.p);
+    const unsigned grid = blocks_for(long(n) * 27, 256);
+    band_codes_kernel<<<grid, 256, 0, stream>>>(n, t->node.p, d.nbr.p, map.p, code.p);
+    band_need_kernel<<<grid, 256, 0, stream>>>(n, p.slots, code.p, need.p);
+    band_halo_kernel<<<BG_CTAS, 256, 0, stream>>>(n, p.slots, need.p, t->node.p, t->push.p, t->hnode.p, t->hcount.p);
+    band_local_kernel<<<grid, 256, 0, stream>>>(n, p.slots, code.p, t->push.p, t->local.p);
+    SGS_CUDA(cudaGetLastError());
+    int count[BG_CTAS];
+    SGS_CUDA(cudaMemcpyAsync(count, t->hcount.p, sizeof(count), cudaMemcpyDeviceToHost, stream));
+    SGS_CUDA(cudaStreamSynchronize(stream));
+    for (int c : count) p.halo = std::max(p.halo, c);
+    if (p.slots + p.halo >= BG_NOWHERE) return;
+    bool ok;
+    if (l > 0)
+      ok = mixed() ? cluster_runs(bandc_group_kernel<float>, bandc_smem<float>(p))
+                   : cluster_runs(bandc_group_kernel<double>, bandc_smem<double>(p));
+    else if (mixed())  // the packed iterate of the V-cycle, the planes of the unit operators
+      ok = cluster_runs(band0_group_kernel<float, true>, band0_smem<float>(p)) &&
+           cluster_runs(band0_group_kernel<float, false>, band0_smem<float>(p));
+    else
+      ok = cluster_runs(band0_group_kernel<double, true>, band0_smem<double>(p)) &&
+           cluster_runs(band0_group_kernel<double, false>, band0_smem<double>(p));
+    if (!ok) return;
+    band[l] = std::move(t);
+  }
+
+  // `count` boundary-band sweeps of level l as one cluster launch; false where
+  // the level has no tables for it (the sweeps then run pass by pass)
+  template <typename T>
+  bool band_group(int l, T* u, const T* b, bool forward, int count, int round) {
+    if (l >= int(band.size()) || !band[l] || (sizeof(T) == 4) != mixed()) return false;
+    if (count <= 0) return true;
+    Level<T>& d = lev<T>(l);
+    const BandTables& t = *band[l];
+    if (l > 0)
+      launch_group(bandc_group_kernel<T>, bandc_smem<T>(t.plan), t.plan, t.node.p, t.local.p, t.push.p, t.hnode.p,
+                   t.hcount.p, d.nbr.p, d.A.p, u, b, d.flags.p, d.N, count, int(forward), round);
+    else if (!u)
+      launch_group(band0_group_kernel<T, true>, band0_smem<T>(t.plan), t.plan, t.node.p, t.local.p, t.push.p,
+                   t.hnode.p, t.hcount.p, d.nbr.p, d.u4.p, nullptr, Edev<T>(), b, d.flags.p, int(d.N), T(P.dx), count, int(forward), round);
+    else
+      launch_group(band0_group_kernel<T, false>, band0_smem<T>(t.plan), t.plan, t.node.p, t.local.p, t.push.p,
+                   t.hnode.p, t.hcount.p, d.nbr.p, nullptr, u, Edev<T>(), b, d.flags.p, int(d.N), T(P.dx), count, int(forward), round);
+    ++launch_counter;
+    return true;
   }
 
   // the packed level-0 iterate with its zero pad block, and the neighbour table naming it
@@ -577,6 +746,7 @@ class Solver {
       upload_level(*L64.back(), h);
       if (first) {
         colour_lists(*L64.back());
+        if (!P.disable_mg && nout() > 1) band_tables(0);
         if (precision == PREC_FP64 && nout() > 1) alloc_packed(*L64.back());
       }
       if (mixed()) {
@@ -701,6 +871,7 @@ class Solver {
       d.spokes.zero(stream);
       d.has_matrix = true;
       stencil_lists(d, h);
+      if (lev > 0 && lev < nout() - 1) band_tables(lev);
       if (ncells > 0) {
         DevBuf<int32_t> dcell;
         dcell.upload(cell_of_slot, stream);
@@ -992,6 +1163,8 @@ class Solver {
   void sweep(int l, T* u, const T* b, bool forward, bool boundary, bool matrix_free = true) {
     Level<T>& d = lev<T>(l);
     if ((boundary ? d.nbound : d.nb) == 0) return;
+    // (level 0's groups leave out the nodes that a pass only clears)
+    if (boundary && l > 0 && band_group<T>(l, u, b, forward, 1, 0)) return;
     if (l == 0 && matrix_free) {
       for (int k = 0; k < 8; ++k) {
         const int c = (boundary ? 8 : 0) + (forward ? k : 7 - k);
@@ -1036,18 +1209,19 @@ class Solver {
   template <typename T>
   void sweeps(int l, T* u, const T* b, bool forward) {
     const bool rr = round_ref();
-    for (int t = 0; t < P.boundary_smoothing; ++t) {
-      sweep<T>(l, u, b, forward, true);
-      if (rr) round3(lev<T>(l), u);
-    }
+    auto boundary = [&] {
+      if (band_group<T>(l, u, b, forward, P.boundary_smoothing, rr ? 1 : 0)) return;
+      for (int t = 0; t < P.boundary_smoothing; ++t) {
+        sweep<T>(l, u, b, forward, true);
+        if (rr) round3(lev<T>(l), u);
+      }
+    };
+    boundary();
     for (int t = 0; t < P.smoothing; ++t) {
       sweep<T>(l, u, b, forward, false);
       if (rr) round3(lev<T>(l), u);
     }
-    for (int t = 0; t < P.boundary_smoothing; ++t) {
-      sweep<T>(l, u, b, forward, true);
-      if (rr) round3(lev<T>(l), u);
-    }
+    boundary();
   }
 
   template <typename T>
