@@ -25,6 +25,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <climits>
 #include <memory>
 #include <string>
 #include <vector>
@@ -117,6 +118,9 @@ __device__ inline bool intersect_box(float3 o, float3 d, float3 bmin, float3 bma
   return *tfar > *tnear;
 }
 
+// whether voxel coordinate i lies outside [0, n) on the side that direction s goes to
+__device__ inline bool left_behind(float i, float s, float n) { return s > 0 ? i >= n : (s < 0 && i < 0); }
+
 // get_next_hit, DDA variant (:214-270): the first voxel above the threshold
 // along the ray and the entry point into it.
 __device__ bool next_hit(const VolumeView& V, float3 o, float3 d, float threshold, float3* hit_pos) {
@@ -146,6 +150,12 @@ __device__ bool next_hit(const VolumeView& V, float3 o, float3 d, float threshol
     else mm = f3(0, 0, 1);
     dis = add(dis, mul(mul(mm, rs), ri));
     ipos = add(ipos, mul(mm, rs));
+    // past the volume on an axis along which the ray moves away from it, every
+    // later voxel reads 0: no hit, unless a negative threshold lets 0 through.
+    // (Without this a ray that misses walked on to RENDER_MAX_STEPS.)
+    if (threshold >= 0 && (left_behind(ipos.x, rs.x, V.box_res.x) || left_behind(ipos.y, rs.y, V.box_res.y) ||
+                           left_behind(ipos.z, rs.z, V.box_res.z)))
+      return false;
   }
   return false;
 }
@@ -237,9 +247,17 @@ __global__ void render_volume_kernel(VolumeView V, Camera C, unsigned W, unsigne
     if (tnear < 0.0f) tnear = 0.0f;
     float3 pos = add(o, scale(d, tnear + 1e-4f));
     const float3 step = scale(d, RENDER_TSTEP);
+    // A sample outside the box adds 0, and a ray never comes back: the march
+    // ends once it has left (its 1025 steps of 0.01 are about 5 to 10 times the
+    // way through the box).  The margin keeps the test clear of the rounding of
+    // sample_world's division.
+    const float3 far = scale(V.box_size, 1.001f);
     for (int i = 0; i < RENDER_MAX_STEPS; ++i) {
       sum += sample_world(V, add(pos, scale(step, rng.next())));
       pos = add(pos, step);
+      if ((step.x >= 0 && pos.x > far.x) || (step.x <= 0 && pos.x < -far.x) || (step.y >= 0 && pos.y > far.y) ||
+          (step.y <= 0 && pos.y < -far.y) || (step.z >= 0 && pos.z > far.z) || (step.z <= 0 && pos.z < -far.z))
+        break;
     }
   }
   sum = float(double(sum) * 1e-2);
@@ -251,17 +269,36 @@ __global__ void render_volume_kernel(VolumeView V, Camera C, unsigned W, unsigne
 
 // ---- the volume from density blocks (volume_renderer.cpp:410-480) ----
 // bounding box of the cells with positive density, per axis
-__global__ void density_bbox_kernel(long ncells, const int* __restrict__ base, const double* __restrict__ rho,
-                                    int* __restrict__ box) {
-  const long t = long(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (t >= ncells || !(rho[t] > 0)) return;
-  const long b = t >> 6;
-  const int e = int(t & 63);
-  const int c[3] = {base[3 * b] + (e >> 4), base[3 * b + 1] + ((e >> 2) & 3), base[3 * b + 2] + (e & 3)};
-  for (int a = 0; a < 3; ++a) {
-    atomicMin(box + a, c[a]);
-    atomicMax(box + 3 + a, c[a] + 1);
+// (grid-stride; one atomic per CTA and bound: one per cell made this kernel
+// the longest of a picture)
+constexpr int BBOX_THREADS = 256, BBOX_BLOCKS = 592;
+__global__ void __launch_bounds__(BBOX_THREADS) density_bbox_kernel(long ncells, const int* __restrict__ base,
+                                                                    const double* __restrict__ rho,
+                                                                    int* __restrict__ box) {
+  __shared__ int sb[6];
+  if (threadIdx.x < 6) sb[threadIdx.x] = threadIdx.x < 3 ? INT_MAX : INT_MIN;
+  __syncthreads();
+  int lo[3] = {INT_MAX, INT_MAX, INT_MAX}, hi[3] = {INT_MIN, INT_MIN, INT_MIN};
+  for (long t = long(blockIdx.x) * BBOX_THREADS + threadIdx.x; t < ncells; t += long(gridDim.x) * BBOX_THREADS) {
+    if (!(rho[t] > 0)) continue;
+    const long b = t >> 6;
+    const int e = int(t & 63);
+    const int c[3] = {base[3 * b] + (e >> 4), base[3 * b + 1] + ((e >> 2) & 3), base[3 * b + 2] + (e & 3)};
+    for (int a = 0; a < 3; ++a) {
+      lo[a] = min(lo[a], c[a]);
+      hi[a] = max(hi[a], c[a] + 1);
+    }
   }
+  for (int a = 0; a < 3; ++a) {
+    const int l = __reduce_min_sync(0xffffffffu, lo[a]), h = __reduce_max_sync(0xffffffffu, hi[a]);
+    if ((threadIdx.x & 31) == 0) {
+      atomicMin(&sb[a], l);
+      atomicMax(&sb[3 + a], h);
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x < 3) atomicMin(box + threadIdx.x, sb[threadIdx.x]);
+  else if (threadIdx.x < 6) atomicMax(box + threadIdx.x, sb[threadIdx.x]);
 }
 
 // voxel = 0 for density 0, else uchar(d * 254) + 1 (d first mapped back from a
@@ -295,7 +332,8 @@ void render_device(const int* base_d, const double* rho_d, long nblocks, const s
   const int init[6] = {1 << 30, 1 << 30, 1 << 30, 0, 0, 0};
   SGS_CUDA(cudaMemcpyAsync(box.p, init, sizeof(init), cudaMemcpyHostToDevice, stream));
   if (ncells)
-    density_bbox_kernel<<<blocks_for(ncells, 256), 256, 0, stream>>>(ncells, base_d, rho_d, box.p);
+    density_bbox_kernel<<<std::min<unsigned>(BBOX_BLOCKS, blocks_for(ncells, BBOX_THREADS)), BBOX_THREADS, 0, stream>>>(
+        ncells, base_d, rho_d, box.p);
   SGS_CUDA(cudaGetLastError());
   int bb[6];
   SGS_CUDA(cudaMemcpyAsync(bb, box.p, sizeof(bb), cudaMemcpyDeviceToHost, stream));
