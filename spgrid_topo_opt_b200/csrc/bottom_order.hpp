@@ -1,0 +1,137 @@
+// Elimination order of the dense bottom inverse.
+//
+// The bottom operator couples a node with its 26 neighbours only.  Its inverse
+// is dense, but while the blocked Gauss-Jordan elimination runs most tiles are
+// still zero if the unknowns are numbered well: a step touches only the tiles
+// its pivot row reaches.  Nodes are numbered by nested dissection (a node plane
+// across the longest extent separates two halves that do not see one another
+// until the plane itself is eliminated, last) and plane by plane inside a part.
+// Parts start on tile boundaries, so that no tile ties two of them together;
+// the padding is identity rows.  Parts of up to LEAF_UNKNOWNS are not cut:
+// below that the padding (half a tile a part on average, which every
+// application of the inverse pays) costs more than the cut saves.
+#pragma once
+#include <algorithm>
+#include <array>
+#include <climits>
+#include <vector>
+
+namespace sgs {
+
+struct BottomOrder {
+  static constexpr int LEAF_UNKNOWNS = 4096;
+  int tile = 128;
+  std::vector<std::array<int, 3>> at;      // node coordinates
+  std::vector<int> pos;                    // node -> its first unknown
+  std::vector<int> pad;                    // identity rows
+  long ld = 0;                             // unknowns and padding, a multiple of tile
+  std::vector<int> list;                   // concatenated: the tiles step K touches, ascending, without K
+  std::vector<int> first;                  // step K's are list[first[K]] .. list[first[K + 1]]
+  std::vector<int> below;                  // how many of them are smaller than K
+
+  void build(int tile_size) {
+    tile = tile_size;
+    pos.assign(at.size(), 0);
+    pad.clear();
+    ld = 0;
+    std::vector<int> all(at.size());
+    for (size_t i = 0; i < all.size(); ++i) all[i] = int(i);
+    dissect(all);
+    symbolic();
+  }
+
+ private:
+  // the axis of the largest extent of `nodes` and its range
+  int longest(const std::vector<int>& nodes, int* lo, int* hi) const {
+    int best = 0;
+    for (int a = 0; a < 3; ++a) {
+      int l = INT_MAX, h = INT_MIN;
+      for (int i : nodes) l = std::min(l, at[size_t(i)][size_t(a)]), h = std::max(h, at[size_t(i)][size_t(a)]);
+      if (a == 0 || h - l > *hi - *lo) best = a, *lo = l, *hi = h;
+    }
+    return best;
+  }
+  void place(std::vector<int>& nodes, int axis) {
+    const int b = (axis + 1) % 3, c = (axis + 2) % 3;
+    std::sort(nodes.begin(), nodes.end(), [&](int i, int j) {
+      const auto &p = at[size_t(i)], &q = at[size_t(j)];
+      if (p[size_t(axis)] != q[size_t(axis)]) return p[size_t(axis)] < q[size_t(axis)];
+      if (p[size_t(b)] != q[size_t(b)]) return p[size_t(b)] < q[size_t(b)];
+      return p[size_t(c)] < q[size_t(c)];
+    });
+    for (int i : nodes) {
+      pos[size_t(i)] = int(ld);
+      ld += 3;
+    }
+    while (ld % tile) pad.push_back(int(ld++));
+  }
+  void dissect(std::vector<int>& nodes) {
+    if (nodes.empty()) return;
+    int lo = 0, hi = 0;
+    const int axis = longest(nodes, &lo, &hi);
+    if (3 * long(nodes.size()) <= LEAF_UNKNOWNS || hi - lo < 2) return place(nodes, axis);
+    // the plane that splits the nodes most evenly
+    std::vector<long> count(size_t(hi - lo + 1), 0);
+    for (int i : nodes) ++count[size_t(at[size_t(i)][size_t(axis)] - lo)];
+    long left = 0, best = LONG_MAX;
+    int cut = lo;
+    for (int p = lo; p <= hi; ++p) {
+      const long right = long(nodes.size()) - left - count[size_t(p - lo)];
+      if (std::max(left, right) < best) best = std::max(left, right), cut = p;
+      left += count[size_t(p - lo)];
+    }
+    std::vector<int> side[3];
+    for (int i : nodes) {
+      const int c = at[size_t(i)][size_t(axis)];
+      side[c < cut ? 0 : (c > cut ? 1 : 2)].push_back(i);
+    }
+    dissect(side[0]);
+    dissect(side[1]);
+    int l2 = 0, h2 = 0;
+    if (!side[2].empty()) place(side[2], longest(side[2], &l2, &h2));
+  }
+  // tiles that each Gauss-Jordan step touches: row K's nonzero tiles S; the step
+  // fills all tiles of S x S
+  void symbolic() {
+    const int nt = int(ld / tile);
+    std::vector<std::vector<char>> on(size_t(nt), std::vector<char>(size_t(nt), 0));
+    if (!at.empty()) {
+      int lo[3], dim[3];
+      for (int a = 0; a < 3; ++a) {
+        int l = INT_MAX, h = INT_MIN;
+        for (const auto& p : at) l = std::min(l, p[size_t(a)]), h = std::max(h, p[size_t(a)]);
+        lo[a] = l - 1;
+        dim[a] = h - l + 3;
+      }
+      std::vector<int> grid(size_t(dim[0]) * dim[1] * dim[2], -1);
+      auto cell = [&](int x, int y, int z) { return (size_t(x - lo[0]) * dim[1] + size_t(y - lo[1])) * dim[2] + size_t(z - lo[2]); };
+      for (size_t i = 0; i < at.size(); ++i) grid[cell(at[i][0], at[i][1], at[i][2])] = int(i);
+      for (size_t i = 0; i < at.size(); ++i)
+        for (int q = 0; q < 27; ++q) {
+          const int j = grid[cell(at[i][0] + q / 9 - 1, at[i][1] + q / 3 % 3 - 1, at[i][2] + q % 3 - 1)];
+          if (j < 0) continue;
+          for (int r : {pos[i] / tile, (pos[i] + 2) / tile})
+            for (int c : {pos[size_t(j)] / tile, (pos[size_t(j)] + 2) / tile}) on[size_t(r)][size_t(c)] = 1;
+        }
+    }
+    list.clear();
+    first.assign(1, 0);
+    below.clear();
+    for (int K = 0; K < nt; ++K) {
+      int low = 0;
+      std::vector<int> S;
+      for (int J = 0; J < nt; ++J)
+        if (J != K && on[size_t(K)][size_t(J)]) {
+          S.push_back(J);
+          low += J < K;
+        }
+      for (int I : S)
+        for (int J : S) on[size_t(I)][size_t(J)] = 1;
+      list.insert(list.end(), S.begin(), S.end());
+      first.push_back(int(list.size()));
+      below.push_back(low);
+    }
+  }
+};
+
+}  // namespace sgs

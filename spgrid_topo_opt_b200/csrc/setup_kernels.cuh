@@ -231,7 +231,8 @@ __global__ void delete_dirichlet_kernel(int nb, const int* __restrict__ coords, 
 // Dense bottom operator over the DOF nodes (nodes with an active spoke), the way
 // Build_CSR_Matrix forms PARDISO's upper triangle (solver/MG/Elasticity_Matrix.cpp:98-161):
 // entry (r,c), r <= c, comes from row r's stencil; Dirichlet rows/columns become identity.
-__global__ void bottom_assemble_kernel(int ndof_nodes, const int* __restrict__ dof_node, const int* __restrict__ node_dof,
+// node_pos: first unknown of a node of the level, -1 without unknowns.
+__global__ void bottom_assemble_kernel(int ndof_nodes, const int* __restrict__ dof_node, const int* __restrict__ node_pos,
                                        const int* __restrict__ coords, const uint32_t* __restrict__ flags,
                                        const uint32_t* __restrict__ spokes, GridView g, const double* __restrict__ A,
                                        long N, double* __restrict__ M, long ld) {
@@ -246,12 +247,12 @@ __global__ void bottom_assemble_kernel(int ndof_nodes, const int* __restrict__ d
     if (!(sp & (1u << q))) continue;
     const long n = g.node(x + q / 9 - 1, y + (q / 3) % 3 - 1, z + q % 3 - 1);
     if (n < 0) continue;
-    const int j = node_dof[n];
+    const int j = node_pos[n];
     if (j < 0) continue;
     const uint32_t nf = flags[n];
     for (int v = 0; v < 3; ++v)
       for (int w = 0; w < 3; ++w) {
-        const long r = 3L * i + v, c = 3L * j + w;
+        const long r = node_pos[gidx] + v, c = j + w;
         if (r > c) continue;
         double val = A[gidx * 243 + q * 9 + v * 3 + w];
         const bool dr = fact && (fl & (DIR_X << v));
@@ -263,129 +264,116 @@ __global__ void bottom_assemble_kernel(int ndof_nodes, const int* __restrict__ d
   }
 }
 
-__global__ void identity_pad_kernel(double* M, long ld, long n0) {
-  long i = n0 + long(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i < ld) M[i * ld + i] = 1.0;
+__global__ void identity_pad_kernel(double* M, long ld, const int* __restrict__ row, int n) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) M[long(row[i]) * ld + row[i]] = 1.0;
 }
 
 // ---------------------------------------------------------------------------
-// Blocked Gauss-Jordan inversion of the (padded) bottom matrix, 64x64 tiles.
-// Sweeping pivot block K: P' = P^-1, A_KJ' = P^-1 A_KJ, A_IJ' = A_IJ - A_IK A_KJ',
-// A_IK' = -A_IK P^-1.  After all pivots the matrix holds its inverse.
-// ---------------------------------------------------------------------------
-constexpr int GJ = 64;
-
-__global__ void __launch_bounds__(256) gj_pivot_kernel(double* M, long ld, int K, double* Pinv, int* bad) {
-  extern __shared__ double sP[];  // 64x65
-  const int t = threadIdx.x;
-  for (int i = t; i < GJ * GJ; i += 256) sP[(i / GJ) * 65 + i % GJ] = M[(long(K) * GJ + i / GJ) * ld + long(K) * GJ + i % GJ];
-  __syncthreads();
-  for (int k = 0; k < GJ; ++k) {
-    const double piv = sP[k * 65 + k];
-    __syncthreads();
-    if (t == 0 && !(piv > 0)) *bad = 1;
-    const double ip = 1.0 / piv;
-    if (t < GJ) sP[k * 65 + t] = (t == k) ? ip : sP[k * 65 + t] * ip;
-    __syncthreads();
-    for (int idx = t; idx < GJ * GJ; idx += 256) {
-      const int i = idx / GJ, j = idx % GJ;
-      if (i == k) continue;
-      const double f = sP[i * 65 + k];
-      if (j == k) continue;
-      sP[i * 65 + j] -= f * sP[k * 65 + j];
-    }
-    __syncthreads();
-    if (t < GJ && t != k) sP[t * 65 + k] = -sP[t * 65 + k] * sP[k * 65 + k];
-    __syncthreads();
-  }
-  for (int i = t; i < GJ * GJ; i += 256) Pinv[i] = sP[(i / GJ) * 65 + i % GJ];
-}
-
-// C = alpha * A(tile) x B(tile) [+ C if accumulate]; tiles addressed by (row tile, col tile)
-// mode 0: row panel  A_KJ <- Pinv * A_KJ        (grid.x = tile J, skip K)
-// mode 1: update     A_IJ <- A_IJ - A_IK*A_KJ   (grid = (J, I), skip K)
-// mode 2: col panel  A_IK <- -A_IK * Pinv       (grid.x = tile I, skip K)
-__global__ void __launch_bounds__(256) gj_tile_kernel(double* M, long ld, int K, const double* __restrict__ Pinv, int mode) {
-  extern __shared__ double sm[];
-  double* sA = sm;             // 64 x 65
-  double* sB = sm + GJ * 65;   // 64 x 65
-  int I, J;
-  const double* srcA;
-  const double* srcB;
-  long lda, ldb;
-  if (mode == 0) {
-    J = blockIdx.x; if (J == K) return; I = K;
-    srcA = Pinv; lda = GJ; srcB = M + long(K) * GJ * ld + long(J) * GJ; ldb = ld;
-  } else if (mode == 1) {
-    J = blockIdx.x; I = blockIdx.y; if (I == K || J == K) return;
-    srcA = M + long(I) * GJ * ld + long(K) * GJ; lda = ld; srcB = M + long(K) * GJ * ld + long(J) * GJ; ldb = ld;
-  } else {
-    I = blockIdx.x; if (I == K) return; J = K;
-    srcA = M + long(I) * GJ * ld + long(K) * GJ; lda = ld; srcB = Pinv; ldb = GJ;
-  }
-  const int t = threadIdx.x;
-  for (int i = t; i < GJ * GJ; i += 256) {
-    sA[(i / GJ) * 65 + i % GJ] = srcA[long(i / GJ) * lda + i % GJ];
-    sB[(i / GJ) * 65 + i % GJ] = srcB[long(i / GJ) * ldb + i % GJ];
-  }
-  __syncthreads();
-  const int ty = t / 16, tx = t % 16;
-  double acc[4][4] = {};
-  for (int k = 0; k < GJ; ++k) {
-    double av[4], bv[4];
-#pragma unroll
-    for (int r = 0; r < 4; ++r) av[r] = sA[(ty + 16 * r) * 65 + k];
-#pragma unroll
-    for (int s = 0; s < 4; ++s) bv[s] = sB[k * 65 + tx + 16 * s];
-#pragma unroll
-    for (int r = 0; r < 4; ++r)
-#pragma unroll
-      for (int s = 0; s < 4; ++s) acc[r][s] += av[r] * bv[s];
-  }
-  double* C = M + long(I) * GJ * ld + long(J) * GJ;
-#pragma unroll
-  for (int r = 0; r < 4; ++r)
-#pragma unroll
-    for (int s = 0; s < 4; ++s) {
-      double* cp = C + long(ty + 16 * r) * ld + tx + 16 * s;
-      if (mode == 0) *cp = acc[r][s];
-      else if (mode == 1) *cp -= acc[r][s];
-      else *cp = -acc[r][s];
-    }
-}
-
-__global__ void gj_store_pivot_kernel(double* M, long ld, int K, const double* __restrict__ Pinv) {
-  for (int i = threadIdx.x; i < GJ * GJ; i += blockDim.x) M[(long(K) * GJ + i / GJ) * ld + long(K) * GJ + i % GJ] = Pinv[i];
-}
-
-// ---------------------------------------------------------------------------
-// Symmetric blocked Gauss-Jordan with 128-wide pivot panels.  The bottom matrix
-// is SPD, and after pivots 0..K-1 tile (I, J) equals the transpose of tile
-// (J, I), negated when exactly one of I, J has been pivoted.  So only the lower
-// tiles (I >= J) are updated; the panels a step needs are gathered from them:
-//   row panel  R_J = A_KJ  (J < K), A_KK, A_JK^T (J > K)
-//   col panel  C_I = A_IK  (I > K), A_KK, -A_KI^T (I < K)
+// Inverse of the bottom matrix: symmetric blocked Gauss-Jordan with 128-wide
+// pivots.  The matrix is SPD, and after pivots 0..K-1 tile (I, J) equals the
+// transpose of tile (J, I), negated when exactly one of I, J has been pivoted.
+// So only the lower tiles (I >= J) are updated; the panels a step needs are
+// gathered from them:
+//   row panel  R_J = A_KJ  (J < K), A_JK^T (J > K)
+//   col panel  C_I = A_IK  (I > K), -A_KI^T (I < K)
 // then T = P^-1 R, lower tiles A_IJ -= C_I T_J, A_IK = -C_I P^-1 (I > K),
 // A_KJ = T_J (J < K), A_KK = P^-1.  After the last pivot the lower tiles hold
-// the lower half of M^-1 and are mirrored.  FP64 GEMM tiles of 128 x 128, a
-// thread computing 8 x 8 entries from k-chunks staged in shared memory.
+// the lower half of M^-1 and are mirrored.  I and J run over the tiles that row
+// K has reached (BottomOrder): with the unknowns in nested-dissection order the
+// steps of the 14739-unknown bottom of a 64^3 box touch about a ninth of the
+// tile products of a full elimination.  FP64 GEMM tiles of 128 x 128.
+// Measured (assembly, inverse and copies): 14739 unknowns 170 -> 35 ms, 20064
+// 409 -> 60 ms, 4287 10 -> 5 ms.  Steps on few tiles are bound by the chain
+// gather, row product, cross update, pivot; the last separators by the DMMA pipe.
 // ---------------------------------------------------------------------------
 constexpr int SGJ = 128, SGJ_K = 16;
 
-__global__ void sgj_gather_kernel(const double* __restrict__ M, long ld, int K, double* __restrict__ R,
-                                  double* __restrict__ Cp, double* __restrict__ P) {
-  const long t = long(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (t >= long(SGJ) * ld) return;
-  const long k0 = long(K) * SGJ;
-  {  // R[r][c], r < 128, c < ld
-    const long r = t / ld, c = t % ld, J = c / SGJ;
-    R[t] = (J <= K) ? M[(k0 + r) * ld + c] : M[c * ld + k0 + r];
+// P = (128 x 128 SPD tile M)^-1 by one CTA of 256 threads, Gauss-Jordan with
+// the tile in registers: thread (ti, tj) holds rows ti + 16 r, columns tj + 16 s.
+// A step publishes the pivot's row and column in shared memory (two buffers, one
+// barrier a step).  Bound by the step's chain (barrier, shared loads, the
+// division, 64 FMAs a thread).
+__global__ void __launch_bounds__(256, 1) sgj_pivot_kernel(const double* __restrict__ M, long ld, double* __restrict__ P,
+                                                           int* bad) {
+  __shared__ double col[2][SGJ], row[2][SGJ];
+  const int ti = threadIdx.x >> 4, tj = threadIdx.x & 15;
+  double a[8][8];
+#pragma unroll
+  for (int r = 0; r < 8; ++r)
+#pragma unroll
+    for (int s = 0; s < 8; ++s) a[r][s] = M[long(ti + 16 * r) * ld + tj + 16 * s];
+#pragma unroll
+  for (int kb = 0; kb < 8; ++kb) {
+    for (int kt = 0; kt < 16; ++kt) {
+      const int p = kt & 1;
+      if (tj == kt)
+#pragma unroll
+        for (int r = 0; r < 8; ++r) col[p][ti + 16 * r] = a[r][kb];
+      if (ti == kt)
+#pragma unroll
+        for (int s = 0; s < 8; ++s) row[p][tj + 16 * s] = a[kb][s];
+      __syncthreads();
+      const double piv = col[p][16 * kb + kt], ip = 1.0 / piv;
+      if (threadIdx.x == 0 && !(piv > 0)) *bad = 1;
+      double rr[8];
+#pragma unroll
+      for (int s = 0; s < 8; ++s) rr[s] = row[p][tj + 16 * s] * ip;
+#pragma unroll
+      for (int r = 0; r < 8; ++r) {
+        const double c = col[p][ti + 16 * r];
+#pragma unroll
+        for (int s = 0; s < 8; ++s) a[r][s] -= c * rr[s];
+        if (tj == kt) a[r][kb] = -c * ip;
+      }
+      if (ti == kt) {
+#pragma unroll
+        for (int s = 0; s < 8; ++s) a[kb][s] = rr[s];
+        if (tj == kt) a[kb][kb] = ip;
+      }
+    }
   }
-  {  // Cp[i][q], i < ld, q < 128
-    const long i = t / SGJ, q = t % SGJ, I = i / SGJ;
-    Cp[t] = (I >= K) ? M[i * ld + k0 + q] : -M[(k0 + q) * ld + i];
+#pragma unroll
+  for (int r = 0; r < 8; ++r)
+#pragma unroll
+    for (int s = 0; s < 8; ++s) P[(ti + 16 * r) * SGJ + tj + 16 * s] = a[r][s];
+}
+
+// panels of step K for the listed tiles J: R [128][ld] and Cp [ld][128]; one CTA
+// (32 x 8 threads) per tile and 32 x 32 part, transposed through shared memory
+__global__ void __launch_bounds__(256) sgj_gather_kernel(const double* __restrict__ M, long ld, int K,
+                                                         const int* __restrict__ list, double* __restrict__ R,
+                                                         double* __restrict__ Cp) {
+  __shared__ double t[32][33];
+  const int J = list[blockIdx.x], pr = int(blockIdx.y >> 2) * 32, pc = int(blockIdx.y & 3) * 32;
+  const bool pivoted = J < K;  // source tile: (K, J) below the diagonal order, else (J, K)
+  const double* src = pivoted ? M + long(K) * SGJ * ld + long(J) * SGJ : M + long(J) * SGJ * ld + long(K) * SGJ;
+  const int x = threadIdx.x, y = threadIdx.y;
+  for (int i = y; i < 32; i += 8) {
+    const double v = src[long(pr + i) * ld + pc + x];
+    t[i][x] = v;
+    if (pivoted) R[long(pr + i) * ld + long(J) * SGJ + pc + x] = v;
+    else Cp[(long(J) * SGJ + pr + i) * SGJ + pc + x] = v;
   }
-  if (P && t < long(SGJ) * SGJ) P[t] = M[(k0 + t / SGJ) * ld + k0 + t % SGJ];
+  __syncthreads();
+  for (int i = y; i < 32; i += 8) {
+    const double v = t[x][i];
+    if (pivoted) Cp[(long(J) * SGJ + pc + i) * SGJ + pr + x] = -v;
+    else R[long(pc + i) * ld + long(J) * SGJ + pr + x] = v;
+  }
+}
+
+// A_KJ = T_J for the first n listed tiles (J < K), A_KK = P (last CTA row)
+__global__ void sgj_store_kernel(double* __restrict__ M, long ld, int K, const int* __restrict__ list, int n,
+                                 const double* __restrict__ T, const double* __restrict__ P) {
+  const int r = blockIdx.y, c = threadIdx.x;  // grid (n + 1, 128), 128 threads
+  double* out = M + (long(K) * SGJ + r) * ld;
+  if (int(blockIdx.x) < n) {
+    const long at = long(list[blockIdx.x]) * SGJ + c;
+    out[at] = T[long(r) * ld + at];
+  } else {
+    out[long(K) * SGJ + c] = P[r * SGJ + c];
+  }
 }
 
 // One FP64 tensor-core MMA (m16n8k8): D = A B + D on a 16 x 8 tile.  With
@@ -402,15 +390,15 @@ __device__ __forceinline__ void dmma_16x8x8(double (&d)[4], const double (&a)[4]
 // C(tile) = alpha * A(tile rows, 0:k) * B(0:k, tile cols) + beta * C(tile) on
 // 128 x 128 tiles: sixteen warps of 32 x 32 (four per SM sub-partition, to hide
 // the MMA latency), k staged through shared memory in chunks of 16, FP64 MMAs.
-// Tiles: SGJ_DENSE (blockIdx.y, blockIdx.x); SGJ_LOWER the tiles I >= J of a
-// square grid (blockIdx.x), leaving out row and column `skip` (none if < 0);
-// SGJ_CROSS the lower tiles of row and column `skip` (blockIdx.x = J for
-// J <= skip, else I).
+// Tiles of the list (ascending): SGJ_ROW (0, list[blockIdx.x]); SGJ_COL
+// (list[blockIdx.x], 0); SGJ_LOWER the pairs I >= J (blockIdx.x), leaving out
+// row and column `skip` (none if < 0); SGJ_CROSS the lower tiles of row and
+// column `skip`.
 constexpr int SGJ_THREADS = 512;          // sixteen warps of 32 x 32 per 128 x 128 tile
 constexpr int SGJ_AS = 20, SGJ_BS = 132;  // padded strides (4 mod 16 doubles): conflict-free fragment loads
 constexpr int SGJ_STAGE = SGJ * SGJ_AS + SGJ_K * SGJ_BS;  // doubles per pipeline stage
 constexpr size_t SGJ_SMEM = 2 * SGJ_STAGE * sizeof(double);
-enum { SGJ_DENSE = 0, SGJ_LOWER = 1, SGJ_CROSS = 2 };
+enum { SGJ_ROW = 0, SGJ_COL = 1, SGJ_LOWER = 2, SGJ_CROSS = 3 };
 
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
   const unsigned s = unsigned(__cvta_generic_to_shared(smem));
@@ -424,7 +412,8 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // chunk c + 1 runs while chunk c is multiplied.
 __global__ void __launch_bounds__(SGJ_THREADS, 1) sgj_gemm_kernel(int k, const double* __restrict__ A, long lda,
                                                           const double* __restrict__ B, long ldb, double* C, long ldc,
-                                                          double alpha, double beta, int mode, int skip) {
+                                                          double alpha, double beta, int mode, int skip,
+                                                          const int* __restrict__ list) {
   extern __shared__ __align__(16) double sg[];
   long I, J;
   if (mode == SGJ_LOWER) {
@@ -432,16 +421,16 @@ __global__ void __launch_bounds__(SGJ_THREADS, 1) sgj_gemm_kernel(int k, const d
     long i = long((sqrt(8.0 * double(t) + 1.0) - 1.0) * 0.5);
     while ((i + 1) * (i + 2) / 2 <= t) ++i;
     while (i * (i + 1) / 2 > t) --i;
-    I = i;
-    J = t - i * (i + 1) / 2;
+    I = list[i];
+    J = list[t - i * (i + 1) / 2];
     if (I == skip || J == skip) return;
   } else if (mode == SGJ_CROSS) {
-    const long b = blockIdx.x;
+    const long b = list[blockIdx.x];
     I = b <= skip ? skip : b;
     J = b <= skip ? b : skip;
   } else {
-    I = blockIdx.y;
-    J = blockIdx.x;
+    I = mode == SGJ_COL ? list[blockIdx.x] : 0;
+    J = mode == SGJ_ROW ? list[blockIdx.x] : 0;
   }
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int wr = (warp >> 2) * 32, wc = (warp & 3) * 32;  // the warp's 32 x 32 sub-tile
@@ -547,15 +536,16 @@ __global__ void sgj_mirror_kernel(double* M, long ld) {
 // the level take b, DOF nodes then get the exact solution x = M^-1 b.
 // ---------------------------------------------------------------------------
 template <typename T>
-__global__ void bottom_gather_kernel(int ndof, const int* __restrict__ dof_node, const T* __restrict__ b, long N,
-                                     double* __restrict__ xb) {
+__global__ void bottom_gather_kernel(int ndof, const int* __restrict__ dof_node, const int* __restrict__ dof_pos,
+                                     const T* __restrict__ b, long N, double* __restrict__ xb) {
   pdl_wait();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= ndof) return;
   long n = dof_node[i];
-  xb[3 * i] = double(b[n]);
-  xb[3 * i + 1] = double(b[n + N]);
-  xb[3 * i + 2] = double(b[n + 2 * N]);
+  double* x = xb + dof_pos[i];
+  x[0] = double(b[n]);
+  x[1] = double(b[n + N]);
+  x[2] = double(b[n + 2 * N]);
 }
 
 // y = M x, one warp per row
@@ -603,15 +593,16 @@ __global__ void __launch_bounds__(1024) gemv32_kernel(const float* __restrict__ 
 }
 
 template <typename T>
-__global__ void bottom_scatter_kernel(int ndof, const int* __restrict__ dof_node, const double* __restrict__ xs,
-                                      T* __restrict__ u, long N) {
+__global__ void bottom_scatter_kernel(int ndof, const int* __restrict__ dof_node, const int* __restrict__ dof_pos,
+                                      const double* __restrict__ xs, T* __restrict__ u, long N) {
   pdl_wait();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= ndof) return;
   long n = dof_node[i];
-  u[n] = T(xs[3 * i]);
-  u[n + N] = T(xs[3 * i + 1]);
-  u[n + 2 * N] = T(xs[3 * i + 2]);
+  const double* x = xs + dof_pos[i];
+  u[n] = T(x[0]);
+  u[n + N] = T(x[1]);
+  u[n + 2 * N] = T(x[2]);
 }
 
 }  // namespace sgs

@@ -30,6 +30,7 @@
 #include "../../include/spgrid_fem.h"
 #include "band.hpp"
 #include "band_group.cuh"
+#include "bottom_order.hpp"
 #include "common.cuh"
 #include "kernels.cuh"
 #include "setup.hpp"
@@ -100,7 +101,10 @@ struct Level {
 struct Bottom {
   int ndof_nodes = 0;
   long n = 0, ld = 0;
-  DevBuf<int> dof_node, node_dof;
+  DevBuf<int> dof_node, dof_pos, node_pos;  // nodes with unknowns, their first unknowns, and those by node
+  BottomOrder order;
+  std::vector<int32_t> ordered_nodes;  // the nodes `order` was made for
+  DevBuf<int> tiles, pad;              // BottomOrder::list and pad on the device
   DevBuf<double> Minv, xb, xs;
   DevBuf<float> Minv32;  // mixed precision: the FP32 V-cycle applies an FP32 copy of Minv
 };
@@ -933,15 +937,11 @@ class Solver {
     std::vector<uint32_t> sp(size_t(d.N));
     if (d.N) SGS_CUDA(cudaMemcpyAsync(sp.data(), d.spokes.p, d.N * 4, cudaMemcpyDeviceToHost, stream));
     SGS_CUDA(cudaStreamSynchronize(stream));
-    std::vector<int32_t> dof_node, node_dof(size_t(d.N), -1);
+    std::vector<int32_t> dof_node;
     for (long i = 0; i < d.N; ++i)
-      if (sp[i] & 0x07ffffffu) {
-        node_dof[i] = int(dof_node.size());
-        dof_node.push_back(int(i));
-      }
+      if (sp[i] & 0x07ffffffu) dof_node.push_back(int(i));
     bottom.ndof_nodes = int(dof_node.size());
     bottom.n = 3L * bottom.ndof_nodes;
-    bottom.ld = ((bottom.n + SGJ - 1) / SGJ) * SGJ;
     const long max_dense = 24576;  // 4.8 GB of FP64
     if (bottom.n > max_dense) {
       char m[160];
@@ -951,8 +951,26 @@ class Solver {
                     bottom.n, max_dense);
       throw CudaError(m, SGS_ERR_INPUT);
     }
-    bottom.dof_node.upload(dof_node, stream);
-    bottom.node_dof.upload(node_dof, stream);
+    if (bottom.ordered_nodes != dof_node || !bottom.dof_node.p) {  // the hierarchy's nodes: once per session
+      BottomOrder& o = bottom.order;
+      const HostLevel& h = P.levels[size_t(nlev() - 1)];
+      o.at.clear();
+      for (int32_t i : dof_node) {
+        const int32_t* c = &h.coords[3 * size_t(i >> 7)];
+        o.at.push_back({c[0] + ((i >> 5) & 3), c[1] + ((i >> 3) & 3), c[2] + (i & 7)});
+      }
+      o.build(SGJ);
+      std::vector<int32_t> node_pos(size_t(d.N), -1);
+      for (size_t k = 0; k < dof_node.size(); ++k) node_pos[size_t(dof_node[k])] = o.pos[k];
+      bottom.dof_node.upload(dof_node, stream);
+      bottom.dof_pos.upload(o.pos, stream);
+      bottom.node_pos.upload(node_pos, stream);
+      bottom.tiles.upload(o.list, stream);
+      bottom.pad.upload(o.pad, stream);
+      SGS_CUDA(cudaStreamSynchronize(stream));
+      bottom.ordered_nodes = dof_node;
+    }
+    bottom.ld = bottom.order.ld;
     bottom.xb.alloc(size_t(bottom.ld));
     bottom.xs.alloc(size_t(bottom.ld));
     bottom.xb.zero(stream);
@@ -961,15 +979,17 @@ class Solver {
     bottom.Minv.alloc(size_t(bottom.ld) * bottom.ld);
     bottom.Minv.zero(stream);
     bottom_assemble_kernel<<<blocks_for(bottom.ndof_nodes, 128), 128, 0, stream>>>(
-        bottom.ndof_nodes, bottom.dof_node.p, bottom.node_dof.p, d.coords.p, d.flags.p, d.spokes.p, d.grid, d.A.p, d.N,
+        bottom.ndof_nodes, bottom.dof_node.p, bottom.node_pos.p, d.coords.p, d.flags.p, d.spokes.p, d.grid, d.A.p, d.N,
         bottom.Minv.p, bottom.ld);
-    if (bottom.ld > bottom.n)
-      identity_pad_kernel<<<blocks_for(bottom.ld - bottom.n, 64), 64, 0, stream>>>(bottom.Minv.p, bottom.ld, bottom.n);
+    if (bottom.pad.n)
+      identity_pad_kernel<<<blocks_for(long(bottom.pad.n), 64), 64, 0, stream>>>(bottom.Minv.p, bottom.ld, bottom.pad.p,
+                                                                                 int(bottom.pad.n));
     SGS_CUDA(cudaGetLastError());
-    invert_dense(bottom.Minv.p, bottom.ld);
+    invert_bottom(bottom.Minv.p, bottom.ld);
     if (mixed()) {
+      // the most that any session's bottom needs (the attribute is the kernel's, not the session's)
       SGS_CUDA(cudaFuncSetAttribute(gemv32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    int(bottom.ld * sizeof(float))));
+                                    int(std::max(bottom.ld, 28672L) * sizeof(float))));
       bottom.Minv32.alloc(bottom.Minv.n);
       convert_kernel<float, double><<<blocks_for(long(bottom.Minv.n), 256), 256, 0, stream>>>(
           bottom.Minv32.p, bottom.Minv.p, long(bottom.Minv.n));
@@ -980,29 +1000,25 @@ class Solver {
     }
   }
 
-  // In-place inverse of the SPD bottom matrix (ld a multiple of SGJ): symmetric
-  // blocked Gauss-Jordan over 128-wide pivots (lower tiles only, see
-  // setup_kernels.cuh); each 128 x 128 pivot block is inverted by the 64-wide
-  // Gauss-Jordan kernels on a second stream, one step ahead: as soon as step K
-  // has updated the row and column of pivot K+1, that block is inverted while
-  // the rest of step K's update runs.
-  void invert_dense(double* M, long ld) {
+  // In-place inverse of the SPD bottom matrix in bottom.order's numbering (ld a
+  // multiple of SGJ): symmetric blocked Gauss-Jordan over 128-wide pivots, each
+  // step on the tiles its pivot row has reached (lower tiles only, see
+  // setup_kernels.cuh).  The pivot blocks are inverted on a second stream, one
+  // step ahead: as soon as step K has updated the row and column of pivot K+1,
+  // that block is inverted while the rest of step K's update runs.
+  void invert_bottom(double* M, long ld) {
     const int nt = int(ld / SGJ);
-    DevBuf<double> R, T, Cp, P[2], pinv;
+    const BottomOrder& o = bottom.order;
+    DevBuf<double> R, T, Cp, P[2];
     R.alloc(size_t(SGJ) * ld);
     T.alloc(size_t(SGJ) * ld);
     Cp.alloc(size_t(SGJ) * ld);
     P[0].alloc(size_t(SGJ) * SGJ);
     P[1].alloc(size_t(SGJ) * SGJ);
-    pinv.alloc(GJ * GJ);
     DevBuf<int> bad;
     bad.alloc(1);
     bad.zero(stream);
-    const size_t tile_smem = 2 * GJ * 65 * sizeof(double);
-    SGS_CUDA(cudaFuncSetAttribute(gj_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(tile_smem)));
     SGS_CUDA(cudaFuncSetAttribute(sgj_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(SGJ_SMEM)));
-    const long nel = long(SGJ) * ld;
-    const size_t row = size_t(ld) * sizeof(double), tile_row = SGJ * sizeof(double);
     // the look-ahead pivot inversion runs beside the update, whose CTAs fill the
     // SMs: its stream has the highest priority so that it takes the first free SM
     cudaStream_t aux;
@@ -1012,48 +1028,44 @@ class Solver {
     cudaEvent_t crossed, inverted;
     SGS_CUDA(cudaEventCreateWithFlags(&crossed, cudaEventDisableTiming));
     SGS_CUDA(cudaEventCreateWithFlags(&inverted, cudaEventDisableTiming));
-    // P <- (diagonal tile K)^-1 on stream st
-    auto invert_pivot = [&](int K, double* Pk, cudaStream_t st) {
-      SGS_CUDA(cudaMemcpy2DAsync(Pk, tile_row, M + size_t(K) * SGJ * ld + size_t(K) * SGJ, row, tile_row, SGJ,
-                                 cudaMemcpyDeviceToDevice, st));
-      for (int k = 0; k < SGJ / GJ; ++k) {
-        gj_pivot_kernel<<<1, 256, GJ * 65 * sizeof(double), st>>>(Pk, SGJ, k, pinv.p, bad.p);
-        gj_tile_kernel<<<SGJ / GJ, 256, tile_smem, st>>>(Pk, SGJ, k, pinv.p, 0);
-        gj_tile_kernel<<<dim3(SGJ / GJ, SGJ / GJ), 256, tile_smem, st>>>(Pk, SGJ, k, pinv.p, 1);
-        gj_tile_kernel<<<SGJ / GJ, 256, tile_smem, st>>>(Pk, SGJ, k, pinv.p, 2);
-        gj_store_pivot_kernel<<<1, 256, 0, st>>>(Pk, SGJ, k, pinv.p);
-      }
+    auto invert_pivot = [&](int K, cudaStream_t st) {
+      sgj_pivot_kernel<<<1, 256, 0, st>>>(M + size_t(K) * SGJ * ld + size_t(K) * SGJ, ld, P[K & 1].p, bad.p);
     };
-    invert_pivot(0, P[0].p, stream);
+    invert_pivot(0, stream);
     for (int K = 0; K < nt; ++K) {
-      double* Pk = P[K & 1].p;
-      if (K > 0) SGS_CUDA(cudaStreamWaitEvent(stream, inverted, 0));
-      sgj_gather_kernel<<<blocks_for(nel, 256), 256, 0, stream>>>(M, ld, K, R.p, Cp.p, nullptr);
-      // T = P^-1 R
-      sgj_gemm_kernel<<<dim3(nt, 1), SGJ_THREADS, SGJ_SMEM, stream>>>(SGJ, Pk, SGJ, R.p, ld, T.p, ld, 1.0, 0.0, SGJ_DENSE, -1);
+      const double* Pk = P[K & 1].p;
+      const int* tiles = bottom.tiles.p + o.first[size_t(K)];
+      const int n = o.first[size_t(K) + 1] - o.first[size_t(K)], low = o.below[size_t(K)];
       const int next = K + 1 < nt ? K + 1 : -1;
-      if (next >= 0) {
-        // the row and column of the next pivot first, then its inverse on the side stream
-        sgj_gemm_kernel<<<nt, SGJ_THREADS, SGJ_SMEM, stream>>>(SGJ, Cp.p, SGJ, T.p, ld, M, ld, -1.0, 1.0, SGJ_CROSS, next);
+      // pivot K+1 is the list's first tile above K if row K has reached it
+      const bool reached = next >= 0 && low < n && o.list[size_t(o.first[size_t(K)] + low)] == next;
+      if (K > 0) SGS_CUDA(cudaStreamWaitEvent(stream, inverted, 0));
+      if (n > 0) {
+        sgj_gather_kernel<<<dim3(unsigned(n), 16), dim3(32, 8), 0, stream>>>(M, ld, K, tiles, R.p, Cp.p);
+        // T = P^-1 R
+        sgj_gemm_kernel<<<n, SGJ_THREADS, SGJ_SMEM, stream>>>(SGJ, Pk, SGJ, R.p, ld, T.p, ld, 1.0, 0.0, SGJ_ROW, -1, tiles);
+        // the row and column of the next pivot first
+        if (reached)
+          sgj_gemm_kernel<<<n, SGJ_THREADS, SGJ_SMEM, stream>>>(SGJ, Cp.p, SGJ, T.p, ld, M, ld, -1.0, 1.0, SGJ_CROSS, next,
+                                                                tiles);
+      }
+      if (next >= 0) {  // then its inverse on the side stream
         SGS_CUDA(cudaEventRecord(crossed, stream));
         SGS_CUDA(cudaStreamWaitEvent(aux, crossed, 0));
-        invert_pivot(next, P[next & 1].p, aux);
+        invert_pivot(next, aux);
         SGS_CUDA(cudaEventRecord(inverted, aux));
       }
-      // the other lower tiles: M -= Cp T
-      sgj_gemm_kernel<<<unsigned(long(nt) * (nt + 1) / 2), SGJ_THREADS, SGJ_SMEM, stream>>>(SGJ, Cp.p, SGJ, T.p, ld, M, ld, -1.0,
-                                                                             1.0, SGJ_LOWER, next);
-      // A_IK = -Cp_I P^-1 below the pivot
-      if (K + 1 < nt)
-        sgj_gemm_kernel<<<dim3(1, nt - K - 1), SGJ_THREADS, SGJ_SMEM, stream>>>(SGJ, Cp.p + size_t(K + 1) * SGJ * SGJ, SGJ, Pk, SGJ,
-                                                                 M + size_t(K + 1) * SGJ * ld + size_t(K) * SGJ, ld,
-                                                                 -1.0, 0.0, SGJ_DENSE, -1);
+      if (n > 0) {
+        // the other lower tiles: M -= Cp T
+        sgj_gemm_kernel<<<unsigned(long(n) * (n + 1) / 2), SGJ_THREADS, SGJ_SMEM, stream>>>(
+            SGJ, Cp.p, SGJ, T.p, ld, M, ld, -1.0, 1.0, SGJ_LOWER, reached ? next : -1, tiles);
+        // A_IK = -Cp_I P^-1 below the pivot
+        if (low < n)
+          sgj_gemm_kernel<<<n - low, SGJ_THREADS, SGJ_SMEM, stream>>>(SGJ, Cp.p, SGJ, Pk, SGJ, M + size_t(K) * SGJ, ld, -1.0,
+                                                                      0.0, SGJ_COL, -1, tiles + low);
+      }
       // A_KJ = T_J left of the pivot, A_KK = P^-1
-      if (K > 0)
-        SGS_CUDA(cudaMemcpy2DAsync(M + size_t(K) * SGJ * ld, row, T.p, row, size_t(K) * SGJ * sizeof(double), SGJ,
-                                   cudaMemcpyDeviceToDevice, stream));
-      SGS_CUDA(cudaMemcpy2DAsync(M + size_t(K) * SGJ * ld + size_t(K) * SGJ, row, Pk, tile_row, tile_row, SGJ,
-                                 cudaMemcpyDeviceToDevice, stream));
+      sgj_store_kernel<<<dim3(unsigned(low + 1), SGJ), SGJ, 0, stream>>>(M, ld, K, tiles, low, T.p, Pk);
     }
     SGS_CUDA(cudaStreamSynchronize(aux));
     cudaEventDestroy(crossed);
@@ -1269,6 +1281,7 @@ class Solver {
     SGS_CUDA(cudaMemcpyAsync(d.u.p, d.b.p, 3 * d.N * sizeof(T), cudaMemcpyDeviceToDevice, stream));
     if (bottom.ndof_nodes > 0) {
       launch(bottom_gather_kernel<T>, blocks_for(bottom.ndof_nodes, 128), 128, 0, bottom.ndof_nodes, bottom.dof_node.p,
+             bottom.dof_pos.p,
                                                                                      d.b.p, d.N, bottom.xb.p);
       if (sizeof(T) == 4 && bottom.Minv32.p)  // the FP32 V-cycle applies the FP32 copy
         launch(gemv32_kernel, blocks_for(bottom.ld, GEMV32_ROWS), 1024, size_t(bottom.ld) * sizeof(float),
@@ -1277,7 +1290,7 @@ class Solver {
         launch(gemv_kernel, blocks_for(bottom.ld * 32, 256), 256, 0, bottom.Minv.p, bottom.ld, bottom.ld, bottom.xb.p,
                bottom.xs.p);
       launch(bottom_scatter_kernel<T>, blocks_for(bottom.ndof_nodes, 128), 128, 0, bottom.ndof_nodes,
-                                                                                      bottom.dof_node.p, bottom.xs.p,
+                                                                                      bottom.dof_node.p, bottom.dof_pos.p, bottom.xs.p,
                                                                                       d.u.p, d.N);
       launch_counter += 3;
     }

@@ -1,0 +1,28 @@
+"""The dense bottom inverse in nested-dissection order (bottom_order.hpp):
+bottoms of several parts with padding between them, against the oracle's exact
+bottom solve.  FP64, relative 1e-10 as test_bottom_solve_and_vcycle."""
+import numpy as np
+import pytest
+
+from oracle import oracle as orc
+from spgrid_topo_opt_b200 import configs, native
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("name", ["box44", "bridge72", "shell96"])
+def test_bottom_solve_in_parts(native_lib, name):
+    if name == "box44":        # 12^3 nodes: two halves and a plane
+        inp = configs.to_inputs(configs.cantilever_box(44, density=(0.2, 1.0), bottom_size=16))
+    elif name == "bridge72":   # 19 x 7 x 13 nodes, supports at four corners
+        inp = configs.to_inputs(configs.bridge(72, 24, 48, density=0.5, bottom_size=20, support_radius=0.06))
+    else:                      # a shell: parts with holes
+        inp = configs.to_inputs(configs.sphere_shell(96, bottom_size=24))
+    o = orc.Oracle(inp, mode=orc.MODE_FP64)
+    with native.Session(inp, precision=native.PRECISION_FP64) as s:
+        top = s.levels - 1
+        fl = s.flags(top)
+        b = np.random.default_rng(3).standard_normal((3, len(fl))) * ((fl & 0x10) != 0)
+        got, want = s.apply(native.OP_BOTTOM, top, b), o.apply(orc.OP_BOTTOM, top, b)
+        assert s.solve(tolerance=1e-2)["bottom_unknowns"] > 4096
+    assert np.abs(got - want).max() <= 1e-10 * np.abs(want).max()
