@@ -28,7 +28,7 @@
 
 namespace sgs {
 
-constexpr int BG_CTAS = 16, BG_THREADS = 512, BG_SLOTS = 512;
+constexpr int BG_CTAS = 16, BG_THREADS = 512, BG_SLOTS = 640;
 constexpr uint32_t BG_OUTSIDE = 0xffffffffu;
 constexpr int BG_NONE = INT32_MIN;  // unused slot
 
@@ -174,7 +174,7 @@ constexpr size_t band0_smem(const BandPlan& p) { return band_smem<T>(p, 8 + 9); 
 template <typename T>
 constexpr size_t bandc_smem(const BandPlan& p) { return band_smem<T>(p, 243 + 9); }
 
-// Level 0, eight threads per node as in gs0_cell4_kernel (thread I the cell of
+// Level 0, eight threads per node as in gs0_cell_kernel (thread I the cell of
 // which the node is corner I).  PACKED: the iterate is u4 (u, E), else the
 // planes of u.  What bounds a pass is its chain: 8 distributed loads, 24
 // dependent FMAs, three rounds of shuffles, the 3x3 update, the barrier.

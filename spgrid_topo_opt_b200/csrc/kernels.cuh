@@ -100,118 +100,207 @@ __device__ __forceinline__ void pdl_wait() {
 }
 
 // ---------------------------------------------------------------------------
-// Level-0 matrix-free operator on one block per CTA (128 threads, one node each;
-// solver/CPU_Kernels/SPGrid_Linear_Elasticity.h:96-344): OP_KU: out = dx*K*u,
-// OP_RES: out = b - dx*K*u.  u of the block plus a one-node halo and E of the
-// cells around it are staged in shared memory; each node sums its 8 cells,
-// g_I = sum_J Kc[I][J] u_J scaled by E_I.  Empty cells (E = 0) are skipped,
-// which saves the work wherever a warp's nodes share them (band edges).
+// Level-0 matrix-free operator (solver/CPU_Kernels/SPGrid_Linear_Elasticity.h:96-344):
+// OP_KU: out = dx*K*u, OP_RES: out = b - dx*K*u, OP_KUP: dx*K*u with Project
+// and the CTA's partial u.(Ku) (the PCG matvec).
+//
+// The trilinear element is evaluated in the basis of the monomials xi^p, p in
+// {0,1}^3, of its reference cube [-1,1]^3, where the energy almost decouples:
+// of the 24 x 24 entries of the element matrix 33 remain (diagonal, the volume
+// terms lambda tr, the shear pairs).  Corner values go to modes and modal
+// forces back to corners by sums and differences along one axis after the
+// other; edges and faces share them.  One thread marches a column of cells
+// along x: it reads a node plane's four corners once for the cells on both
+// sides, and hands its corner forces to the nodes through shared memory, plane
+// by plane.  About 160 operations a cell, against 576 FMAs a node and 24 shared
+// loads a node and cell in the nodal form.
+// Two blocks per CTA of 96 threads (2 x 45 columns of cells, the block's 4 x 8
+// and one layer below): 90 of 96 lanes work where one block would leave 19 of
+// 64 idle.  Cells without material (E = 0) skip the modal part.
+// PACKED: the iterate is the record u4 = (u, E) with the neighbour table nbrz
+// (a zero pad block for missing blocks), else the planes of u, E and nbr (-1).
+// Bound by shared-memory bandwidth (66 KB a block in FP64) and, in FP64, the FMA
+// pipe.  At 1024^3 (340713 blocks): FP64 matvec 2240 -> 2169 us, FP32 residual
+// 1348 -> 1188 us (nodal form -> this).
 // ---------------------------------------------------------------------------
-enum { OP_KU = 0, OP_RES = 1, OP_KUP = 2 };  // OP_KUP: K u with Project, and the CTA's partial u.(Ku)
+enum { OP_KU = 0, OP_RES = 1, OP_KUP = 2 };
 
-// halo geometry: nodes [-1,4]x[-1,4]x[-1,8] (6x6x10), cells [-1,3]x[-1,3]x[-1,7] (5x5x9).
-// In shared memory a y-row of the halo starts every HSY = 24 entries: a warp
-// reads 4 consecutive rows of 8 consecutive z at once, and with the row starts
-// at 0, 24, 48, 72 (mod 32 banks: 0, 24, 16, 8) those 32 words fall in distinct
-// banks (FP32), or in distinct bank pairs per half-warp (FP64).  Rows of 10
-// entries would put rows y and y+3 on the same banks.
+// halo geometry: nodes [-1,4]x[-1,4]x[-1,8] (6x6x10), cells [-1,3]x[-1,3]x[-1,7] (5x5x9)
 constexpr int HU = 360, HE = 225;
-constexpr int HSY = 24;
-constexpr int HSX = 5 * HSY + 10, HN = 6 * HSX;   // node halo: x-plane stride, entries
-constexpr int ESX = 4 * HSY + 9, HEN = 5 * ESX;   // cell halo
+constexpr int MODAL_THREADS = 96, MODAL_BLOCKS = 2, MODAL_COLS = 45;
 
-template <typename T, int OP>
-__global__ void __launch_bounds__(128) level0_op_kernel(const int* __restrict__ block_list, int nblocks,
-                                                        const int* __restrict__ nbr, const T* __restrict__ E,
-                                                        const T* u, const T* __restrict__ b, T* __restrict__ out,
-                                                        long N, T dx, const uint32_t* __restrict__ flags,
-                                                        double* __restrict__ part) {
+// dx/16 times the Lame parameters and their modal combinations
+template <typename T>
+struct ModalCoef {
+  T m, l, A, L, M, B;  // mu, lambda, (3 mu + lambda)/3, lambda/3, mu/3, (4 mu + lambda)/9
+  void set(double mu, double la, double dx) {
+    const double mm = mu * dx / 16, ll = la * dx / 16;
+    m = T(mm), l = T(ll), A = T((3 * mm + ll) / 3), L = T(ll / 3), M = T(mm / 3), B = T((4 * mm + ll) / 9);
+  }
+};
+
+// one value to shared memory with cp.async (zero where !on): a thread's whole
+// share of a halo is in flight at once
+template <typename T>
+__device__ __forceinline__ void stage_async(T* smem, const T* gmem, bool on) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n" ::"r"(unsigned(__cvta_generic_to_shared(smem))), "l"(gmem),
+               "n"(int(sizeof(T))), "r"(on ? int(sizeof(T)) : 0)
+               : "memory");
+}
+
+template <typename T, int OP, bool PACKED>
+__global__ void __launch_bounds__(MODAL_THREADS, sizeof(T) == 8 ? 5 : 8) level0_modal_kernel(
+    int nblocks, const int* __restrict__ nbr, const T* __restrict__ E, const T* __restrict__ u,
+    const typename Pack4<T>::type* __restrict__ u4, const T* __restrict__ b, T* __restrict__ out, long N,
+    ModalCoef<T> K, const uint32_t* __restrict__ flags, double* __restrict__ part) {
+  constexpr int BUFS = sizeof(T) == 8 ? 1 : 2;  // exchange buffers: one more barrier a plane, but more CTAs, in FP64
+  __shared__ T su[MODAL_BLOCKS][3][HU];
+  __shared__ T sE[MODAL_BLOCKS][HE];
+  __shared__ T sx[BUFS][12][MODAL_THREADS];
+  __shared__ int snb[MODAL_BLOCKS * 27];
+  const int t = threadIdx.x;
+  const int b0 = blockIdx.x * MODAL_BLOCKS;
+  if (t < MODAL_BLOCKS * 27) snb[t] = b0 + t / 27 < nblocks ? nbr[long(b0) * 27 + t] : -1;
   pdl_wait();
-  __shared__ T su[3][HN];
-  __shared__ T sE[HEN];
-  __shared__ int snb[27];
-  const int bi = block_list ? block_list[blockIdx.x] : blockIdx.x;
-  if (bi >= 0 && threadIdx.x < 27) snb[threadIdx.x] = nbr[long(bi) * 27 + threadIdx.x];
   __syncthreads();
-  // stage u halo
-  for (int h = threadIdx.x; h < HU; h += 128) {
-    const int sx = h / 60, sy = (h / 10) % 6, sz = h % 10;
-    const int lx = sx - 1, ly = sy - 1, lz = sz - 1;
+  for (int h2 = t; h2 < MODAL_BLOCKS * HU; h2 += MODAL_THREADS) {
+    const int k = h2 / HU, h = h2 % HU;
+    const int sx_ = h / 60, sy = (h / 10) % 6, sz = h % 10;
+    const int lx = sx_ - 1, ly = sy - 1, lz = sz - 1;
     const int dxb = lx < 0 ? 0 : (lx > 3 ? 2 : 1), dyb = ly < 0 ? 0 : (ly > 3 ? 2 : 1), dzb = lz < 0 ? 0 : (lz > 7 ? 2 : 1);
-    const int nb = snb[dxb * 9 + dyb * 3 + dzb];
-    T a = 0, bb = 0, c = 0;
-    if (nb >= 0) {
-      const long idx = long(nb) * 128 + ((lx & 3) << 5) + ((ly & 3) << 3) + (lz & 7);
-      a = u[idx];
-      bb = u[idx + N];
-      c = u[idx + 2 * N];
+    const int nb = snb[k * 27 + dxb * 9 + dyb * 3 + dzb];
+    const long i = nb < 0 ? 0 : long(nb) * 128 + ((lx & 3) << 5) + ((ly & 3) << 3) + (lz & 7);
+    const bool cell = sx_ < 5 && sy < 5 && sz < 9;
+    T* ce = &sE[k][cell ? (sx_ * 5 + sy) * 9 + sz : 0];
+    if (PACKED) {
+      const T* r = reinterpret_cast<const T*>(u4 + i);
+      stage_async(&su[k][0][h], r, nb >= 0);
+      stage_async(&su[k][1][h], r + 1, nb >= 0);
+      stage_async(&su[k][2][h], r + 2, nb >= 0);
+      if (cell) stage_async(ce, r + 3, nb >= 0);
+    } else {
+      stage_async(&su[k][0][h], u + i, nb >= 0);
+      stage_async(&su[k][1][h], u + i + N, nb >= 0);
+      stage_async(&su[k][2][h], u + i + 2 * N, nb >= 0);
+      if (cell) stage_async(ce, E + i, nb >= 0);
     }
-    const int s = sx * HSX + sy * HSY + sz;
-    su[0][s] = a;
-    su[1][s] = bb;
-    su[2][s] = c;
   }
-  for (int h = threadIdx.x; h < HE; h += 128) {
-    const int sx = h / 45, sy = (h / 9) % 5, sz = h % 9;
-    const int lx = sx - 1, ly = sy - 1, lz = sz - 1;
-    const int dxb = lx < 0 ? 0 : 1, dyb = ly < 0 ? 0 : 1, dzb = lz < 0 ? 0 : 1;
-    const int nb = snb[dxb * 9 + dyb * 3 + dzb];
-    sE[sx * ESX + sy * HSY + sz] = nb >= 0 ? E[long(nb) * 128 + ((lx & 3) << 5) + ((ly & 3) << 3) + (lz & 7)] : T(0);
-  }
+  asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
   __syncthreads();
-  const int e = threadIdx.x;
-  const int x = e >> 5, y = (e >> 3) & 3, z = e & 7;
-  const long gidx = long(bi) * 128 + e;
-  T f0 = 0, f1 = 0, f2 = 0;
+  const int blk = t >= MODAL_COLS ? 1 : 0, col = min(t - blk * MODAL_COLS, MODAL_COLS - 1);  // lanes 90..95 idle along
+  const T* un = &su[blk][0][(col / 9) * 10 + col % 9];
+  const T* ec = &sE[blk][col];
+  // modes 1, z, y, yz of a node plane's face
+  auto face = [&](int plane, T (&m)[4][3]) {
 #pragma unroll
-  for (int I = 0; I < 8; ++I) {
-    const int Ix = I >> 2, Iy = (I >> 1) & 1, Iz = I & 1;
-    const int cx = x - Ix, cy = y - Iy, cz = z - Iz;  // cell, in [-1,3]x[-1,3]x[-1,7]
-    const T Ec = sE[(cx + 1) * ESX + (cy + 1) * HSY + (cz + 1)];
-    if (Ec == T(0)) continue;
-    T g0 = 0, g1 = 0, g2 = 0;
-#pragma unroll
-    for (int J = 0; J < 8; ++J) {
-      const int nx = cx + (J >> 2) + 1, ny = cy + ((J >> 1) & 1) + 1, nz = cz + (J & 1) + 1;
-      const int h = nx * HSX + ny * HSY + nz;
-      const T ux = su[0][h], uy = su[1][h], uz = su[2][h];
-      const int k = (I * 8 + J) * 9;
-      g0 += kc<T>(k + 0) * ux + kc<T>(k + 1) * uy + kc<T>(k + 2) * uz;
-      g1 += kc<T>(k + 3) * ux + kc<T>(k + 4) * uy + kc<T>(k + 5) * uz;
-      g2 += kc<T>(k + 6) * ux + kc<T>(k + 7) * uy + kc<T>(k + 8) * uz;
+    for (int c = 0; c < 3; ++c) {
+      const T* p = un + c * HU + plane * 60;
+      const T v00 = p[0], v01 = p[1], v10 = p[10], v11 = p[11];
+      const T s0 = v00 + v01, s1 = v10 + v11, d0 = v01 - v00, d1 = v11 - v10;
+      m[0][c] = s0 + s1;
+      m[1][c] = d0 + d1;
+      m[2][c] = s1 - s0;
+      m[3][c] = d1 - d0;
     }
-    f0 += Ec * g0;
-    f1 += Ec * g1;
-    f2 += Ec * g2;
-  }
-  f0 *= dx;
-  f1 *= dx;
-  f2 *= dx;
-  if (OP == OP_KU) {
-    out[gidx] = f0;
-    out[gidx + N] = f1;
-    out[gidx + 2 * N] = f2;
-  } else if (OP == OP_RES) {
-    out[gidx] = b[gidx] - f0;
-    out[gidx + N] = b[gidx + N] - f1;
-    out[gidx + 2 * N] = b[gidx + 2 * N] - f2;
-  } else {
-    // the PCG matvec q = K s: Dirichlet components zeroed, and s.q summed per CTA
-    const uint32_t fl = flags[gidx];
-    if (fl & DIR_X) f0 = 0;
-    if (fl & DIR_Y) f1 = 0;
-    if (fl & DIR_Z) f2 = 0;
-    out[gidx] = f0;
-    out[gidx + N] = f1;
-    out[gidx + 2 * N] = f2;
-    const int hc = (x + 1) * HSX + (y + 1) * HSY + (z + 1);
-    double d = double(su[0][hc]) * double(f0) + double(su[1][hc]) * double(f1) + double(su[2][hc]) * double(f2);
+  };
+  T P[4][3], H[4][3];  // the last plane's modes; the modal forces on it from the cell behind
+  face(0, P);
 #pragma unroll
-    for (int o = 16; o; o >>= 1) d += __shfl_down_sync(0xffffffffu, d, o);
-    __shared__ double sd[4];
-    if ((threadIdx.x & 31) == 0) sd[threadIdx.x >> 5] = d;
+  for (int k = 0; k < 4; ++k) H[k][0] = H[k][1] = H[k][2] = T(0);
+  double dot = 0;
+#pragma unroll 1
+  for (int x = 0; x < 5; ++x) {  // cell x - 1, between node planes x - 1 and x (own planes are 1..4 of the halo)
+    T Q[4][3];
+    face(x + 1, Q);
+    const T e = ec[x * MODAL_COLS];
+    if (e != T(0)) {
+      T D[4][3], S1[3], S2[3], S3[3];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        S1[c] = P[1][c] + Q[1][c];
+        S2[c] = P[2][c] + Q[2][c];
+        S3[c] = P[3][c] + Q[3][c];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) D[k][c] = Q[k][c] - P[k][c];
+      }
+      const T m = e * K.m, l = e * K.l, A = e * K.A, L = e * K.L, M = e * K.M, B = e * K.B;
+      T G0[3], G1[3], G2[3], F1[3], F2[3], F3[3];  // forces of D[0..2], S1..S3
+      const T lt = l * (D[0][0] + S2[1] + S1[2]), m2 = m + m;
+      G0[0] = fma(m2, D[0][0], lt);
+      F2[1] = fma(m2, S2[1], lt);
+      F1[2] = fma(m2, S1[2], lt);
+      G0[1] = F2[0] = m * (D[0][1] + S2[0]);
+      G0[2] = F1[0] = m * (D[0][2] + S1[0]);
+      F2[2] = F1[1] = m * (S2[2] + S1[1]);
+      G1[0] = fma(A, D[1][0], L * S3[1]);
+      F3[1] = fma(A, S3[1], L * D[1][0]);
+      G1[2] = fma(A, D[1][2], L * D[2][1]);
+      G2[1] = fma(A, D[2][1], L * D[1][2]);
+      G2[0] = fma(A, D[2][0], L * S3[2]);
+      F3[2] = fma(A, S3[2], L * D[2][0]);
+      const T q = D[1][1] + S3[0] + D[2][2];
+      G1[1] = M * (D[1][1] + q);
+      F3[0] = M * (S3[0] + q);
+      G2[2] = M * (D[2][2] + q);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const T G3 = B * D[3][c];
+        H[0][c] -= G0[c];
+        H[1][c] += F1[c] - G1[c];
+        H[2][c] += F2[c] - G2[c];
+        H[3][c] += F3[c] - G3;
+        P[0][c] = G0[c];  // the next plane's share, kept in P while H is handed out
+        P[1][c] = F1[c] + G1[c];
+        P[2][c] = F2[c] + G2[c];
+        P[3][c] = F3[c] + G3;
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) P[k][0] = P[k][1] = P[k][2] = T(0);
+    }
+    if (x > 0) {  // plane x - 1 of the block is complete: corner forces to the nodes
+      T(*ex)[MODAL_THREADS] = sx[x & (BUFS - 1)];
+      if (BUFS == 1) __syncthreads();
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const T e0 = H[0][c] - H[1][c], e1 = H[0][c] + H[1][c], o0 = H[2][c] - H[3][c], o1 = H[2][c] + H[3][c];
+        ex[c][t] = e0 - o0;
+        ex[3 + c][t] = e1 - o1;
+        ex[6 + c][t] = e0 + o0;
+        ex[9 + c][t] = e1 + o1;
+      }
+      __syncthreads();
+      const int c = t >> 5, y = (t >> 3) & 3, z = t & 7;  // warp c sums component c of the plane's 32 nodes
+#pragma unroll
+      for (int k = 0; k < MODAL_BLOCKS; ++k) {
+        if (b0 + k >= nblocks) continue;
+        const int q = k * MODAL_COLS + (y + 1) * 9 + z + 1;  // the column whose min corner is the node
+        T f = (ex[c][q] + ex[3 + c][q - 1]) + (ex[6 + c][q - 9] + ex[9 + c][q - 10]);
+        const long node = long(b0 + k) * 128 + (x - 1) * 32 + (t & 31), g = node + c * N;
+        if (OP == OP_RES) {
+          f = b[g] - f;
+        } else if (OP == OP_KUP) {
+          if (flags[node] & (DIR_X << c)) f = 0;
+          dot += double(su[k][c][x * 60 + (y + 1) * 10 + z + 1]) * double(f);
+        }
+        out[g] = f;
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        H[k][c] = P[k][c];
+        P[k][c] = Q[k][c];
+      }
+  }
+  if (OP == OP_KUP) {
+#pragma unroll
+    for (int o = 16; o; o >>= 1) dot += __shfl_down_sync(0xffffffffu, dot, o);
+    __shared__ double sd[3];
+    if ((t & 31) == 0) sd[t >> 5] = dot;
     __syncthreads();
-    if (threadIdx.x == 0) part[blockIdx.x] = (sd[0] + sd[1]) + (sd[2] + sd[3]);
+    if (t == 0) part[blockIdx.x] = (sd[0] + sd[1]) + sd[2];
   }
 }
 
@@ -583,62 +672,6 @@ __global__ void __launch_bounds__(128) gs0_cell4_kernel(const int* __restrict__ 
   if (fy) v1 = 0;
   if (fz) v2 = 0;
   u4[g] = Pack4<T>::make(v0, v1, v2, Ec);  // thread 0: the node's own cell
-}
-
-// level0_op_kernel<T, OP_RES> on the packed iterate: r = b - dx K u
-template <typename T>
-__global__ void __launch_bounds__(128) level0_res4_kernel(int nblocks, const int* __restrict__ nbrz,
-                                                          const typename Pack4<T>::type* __restrict__ u4,
-                                                          const T* __restrict__ b, T* __restrict__ out, long N, T dx) {
-  pdl_wait();
-  __shared__ T su[3][HN];
-  __shared__ T sE[HN];
-  __shared__ int snb[27];
-  const int bi = blockIdx.x;
-  KcReg<T> K;
-  K.load();
-  if (threadIdx.x < 27) snb[threadIdx.x] = nbrz[long(bi) * 27 + threadIdx.x];
-  __syncthreads();
-  for (int h = threadIdx.x; h < HU; h += 128) {
-    const int sx = h / 60, sy = (h / 10) % 6, sz = h % 10;
-    const int lx = sx - 1, ly = sy - 1, lz = sz - 1;
-    const int dxb = lx < 0 ? 0 : (lx > 3 ? 2 : 1), dyb = ly < 0 ? 0 : (ly > 3 ? 2 : 1), dzb = lz < 0 ? 0 : (lz > 7 ? 2 : 1);
-    const int nb = snb[dxb * 9 + dyb * 3 + dzb];  // the zero pad block where there is none
-    const auto v = u4[long(nb) * 128 + ((lx & 3) << 5) + ((ly & 3) << 3) + (lz & 7)];
-    const int s = sx * HSX + sy * HSY + sz;
-    su[0][s] = v.x;
-    su[1][s] = v.y;
-    su[2][s] = v.z;
-    sE[s] = v.w;
-  }
-  __syncthreads();
-  const int e = threadIdx.x;
-  const int x = e >> 5, y = (e >> 3) & 3, z = e & 7;
-  const long gidx = long(bi) * 128 + e;
-  T f0 = 0, f1 = 0, f2 = 0;
-#pragma unroll
-  for (int I = 0; I < 8; ++I) {
-    const int Ix = I >> 2, Iy = (I >> 1) & 1, Iz = I & 1;
-    const int cx = x - Ix, cy = y - Iy, cz = z - Iz;  // cell = its min-corner node, in the halo
-    const T Ec = sE[(cx + 1) * HSX + (cy + 1) * HSY + (cz + 1)];
-    if (Ec == T(0)) continue;
-    T g0 = 0, g1 = 0, g2 = 0;
-#pragma unroll
-    for (int J = 0; J < 8; ++J) {
-      const int nx = cx + (J >> 2) + 1, ny = cy + ((J >> 1) & 1) + 1, nz = cz + (J & 1) + 1;
-      const int h = nx * HSX + ny * HSY + nz;
-      const T ux = su[0][h], uy = su[1][h], uz = su[2][h];
-      g0 += K(I, J, 0, 0) * ux + K(I, J, 0, 1) * uy + K(I, J, 0, 2) * uz;
-      g1 += K(I, J, 1, 0) * ux + K(I, J, 1, 1) * uy + K(I, J, 1, 2) * uz;
-      g2 += K(I, J, 2, 0) * ux + K(I, J, 2, 1) * uy + K(I, J, 2, 2) * uz;
-    }
-    f0 += Ec * g0;
-    f1 += Ec * g1;
-    f2 += Ec * g2;
-  }
-  out[gidx] = b[gidx] - f0 * dx;
-  out[gidx + N] = b[gidx + N] - f1 * dx;
-  out[gidx + 2 * N] = b[gidx + 2 * N] - f2 * dx;
 }
 
 // ---------------------------------------------------------------------------

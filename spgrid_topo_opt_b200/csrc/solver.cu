@@ -1147,14 +1147,22 @@ class Solver {
     ++launch_counter;
   }
 
+  static unsigned modal_grid(int nb) { return blocks_for(nb, MODAL_BLOCKS); }
+  template <typename T>
+  ModalCoef<T> modal_coef() const {
+    ModalCoef<T> k;
+    k.set(P.mu0, P.lambda0, P.dx);
+    return k;
+  }
+
   // out = dx K u (OP_KU), b - dx K u (OP_RES) or the projected PCG matvec with
   // per-block partial products u.out in red (OP_KUP) over all level-0 blocks
   template <typename T, int OP>
   void level0(const T* u, const T* b, T* out) {
     Level<T>& d = lev<T>(0);
     if (d.nb <= 0) return;
-    launch(level0_op_kernel<T, OP>, d.nb, 128, 0, nullptr, d.nb, d.nbr.p, Edev<T>(), u, b, out, d.N, T(P.dx),
-           d.flags.p, red.p);
+    launch(level0_modal_kernel<T, OP, false>, modal_grid(d.nb), MODAL_THREADS, 0, d.nb, d.nbr.p, Edev<T>(), u, nullptr, b,
+           out, d.N, modal_coef<T>(), d.flags.p, red.p);
     ++launch_counter;
   }
 
@@ -1386,7 +1394,8 @@ class Solver {
       }
     }
     if (OP != OP_RES) throw CudaError("K u on the packed iterate runs on the tensor-core kernel only", SGS_ERR_INPUT);
-    launch(level0_res4_kernel<T>, d.nb, 128, 0, d.nb, d.nbrz.p, d.u4.p, b, out, d.N, T(P.dx));
+    launch(level0_modal_kernel<T, OP_RES, true>, modal_grid(d.nb), MODAL_THREADS, 0, d.nb, d.nbrz.p, nullptr, nullptr,
+           d.u4.p, b, out, d.N, modal_coef<T>(), nullptr, nullptr);
     ++launch_counter;
   }
 
@@ -2133,7 +2142,7 @@ void Solver::record_iteration() {
   launch(axpy_pair_kernel, PAIR_BLOCKS, RED_THREADS, 0, s.p, scal.p, 4, s.p, q.p, N0(),
          round_ref() ? 1 : 0, l0.flags.p);                               // s = beta*s + z
   level0<double, OP_KUP>(s.p, nullptr, q.p);                             // q = K s, Project, s.q partials
-  launch(finish_reduce_kernel, 1, FIN_THREADS, 0, red.p, l0.nb, 0, scal.p, 1);       // alpha
+  launch(finish_reduce_kernel, 1, FIN_THREADS, 0, red.p, int(modal_grid(l0.nb)), 0, scal.p, 1);  // alpha
   launch(cg_update_pair_kernel, PAIR_BLOCKS, RED_THREADS, 0, x.p, s.p, f.p, q.p, scal.p, l0.flags.p, l0.N,
          round_ref() ? 1 : 0, (mixed() && !P.disable_mg) ? L32[0]->b.p : (float*)nullptr, red.p);
   launch(finish_reduce_kernel, 1, FIN_THREADS, 0, red.p, PAIR_BLOCKS, 1, scal.p, 4);  // |r|_inf, rho_old
