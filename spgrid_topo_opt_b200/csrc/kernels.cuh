@@ -566,21 +566,27 @@ __global__ void __launch_bounds__(128, MINB) gs0_list4_kernel(const int* __restr
   u4[g] = Pack4<T>::make(v0, v1, v2, Ec[0]);  // corner I = 0: the node's own cell
 }
 
-// gs0_list4_kernel for the short passes of the boundary band (about 10^3
-// nodes): those are bound by one thread's chain of dependent loads, so eight
-// threads share a node, thread I taking the cell of which the node is corner I.
+// The colour pass for few nodes (a boundary band, a small level: up to
+// GS_CELL_NODES): such a pass is bound by one thread's chain of dependent loads
+// and its 600 FMAs, so eight threads share a node, thread I taking the cell of
+// which the node is corner I.
 // The Q1 element is symmetric under reflections, K(I, J) = S K(0, I^J) S with S
 // = diag(-1 on the axes where I has its bit) (checked on the host at set-up);
 // looping over J' = I^J keeps the coefficients K(0, J') compile-time register
 // selections while the corner J a thread reads varies with I.  Per thread: 8
 // gathers and 72 FMA; the cells' E g and diagonal blocks are summed over the
 // eight threads with shuffles and thread 0 updates the node.  Same products as
-// gs0_list4_kernel, summed in another order.
-template <typename T>
-__global__ void __launch_bounds__(128) gs0_cell4_kernel(const int* __restrict__ list, int n,
-                                                        const int* __restrict__ nbrz,
-                                                        typename Pack4<T>::type* u4, const T* __restrict__ b,
-                                                        const uint32_t* __restrict__ flags, int N, T dx) {
+// gs0_list4_kernel, summed in another order.  PACKED: on u4 with nbrz, else on
+// the planes of u with E and nbr (-1 for missing blocks).
+// Both sides of GS_CELL_NODES: 614 nodes a pass (FP64, planes) 59 -> 26 us a sweep against a thread per
+// node, 1584 nodes 7.4 -> 4.7 us a pass; 15925 nodes (FP32) 33 against 44 us a sweep the other way.
+constexpr int GS_CELL_NODES = 6144;
+template <typename T, bool PACKED>
+__global__ void __launch_bounds__(128) gs0_cell_kernel(const int* __restrict__ list, int n,
+                                                       const int* __restrict__ nbr,
+                                                       typename Pack4<T>::type* u4, T* u, const T* __restrict__ E,
+                                                       const T* __restrict__ b,
+                                                       const uint32_t* __restrict__ flags, int N, T dx) {
   using V = typename Pack4<T>::type;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int k = t >> 3, I = t & 7;  // groups of 8 threads never straddle a warp
@@ -601,23 +607,38 @@ __global__ void __launch_bounds__(128) gs0_cell4_kernel(const int* __restrict__ 
   const int sx[2] = {9, (x1 < 0 ? 0 : (x1 > 3 ? 2 : 1)) * 9}, lx[2] = {(x & 3) << 5, (x1 & 3) << 5};
   const int sy[2] = {3, (y1 < 0 ? 0 : (y1 > 3 ? 2 : 1)) * 3}, ly[2] = {(y & 3) << 3, (y1 & 3) << 3};
   const int sz[2] = {1, z1 < 0 ? 0 : (z1 > 7 ? 2 : 1)}, lz[2] = {z & 7, z1 & 7};
-  const int* nb = nbrz + long(bi) * 27;
+  const int* nb = nbr + long(bi) * 27;
   int idx[8];
 #pragma unroll
   for (int Jp = 0; Jp < 8; ++Jp) {
     const int a = Jp >> 2, c = (Jp >> 1) & 1, d = Jp & 1;
-    idx[Jp] = (__ldg(nb + sx[a] + sy[c] + sz[d]) << 7) + lx[a] + ly[c] + lz[d];
+    const int k27 = __ldg(nb + sx[a] + sy[c] + sz[d]);
+    idx[Jp] = !PACKED && k27 < 0 ? -1 : (k27 << 7) + lx[a] + ly[c] + lz[d];
+  }
+  T Ec = 0;  // the cell's min corner carries its E: J = 0, so J' = I
+  if (!PACKED) {
+    int at = idx[0];
+#pragma unroll
+    for (int Jp = 1; Jp < 8; ++Jp)
+      if (Jp == I) at = idx[Jp];
+    Ec = (raw < 0 || at < 0) ? T(0) : E[at];
   }
   KcReg<T> K;
   K.load();
   pdl_wait();
   if (raw < 0) {
     if (I == 0) {
-      V v = u4[g];
-      if (fx) v.x = T(0);
-      if (fy) v.y = T(0);
-      if (fz) v.z = T(0);
-      u4[g] = v;
+      if (PACKED) {
+        V v = u4[g];
+        if (fx) v.x = T(0);
+        if (fy) v.y = T(0);
+        if (fz) v.z = T(0);
+        u4[g] = v;
+      } else {
+        if (fx) u[g] = T(0);
+        if (fy) u[g + N] = T(0);
+        if (fz) u[g + 2 * N] = T(0);
+      }
     }
     return;
   }
@@ -627,16 +648,23 @@ __global__ void __launch_bounds__(128) gs0_cell4_kernel(const int* __restrict__ 
     asm volatile("prefetch.global.L1 [%0];" ::"l"(b + g + 2 * N));
   }
   const T s0 = Ix ? T(-1) : T(1), s1 = Iy ? T(-1) : T(1), s2 = Iz ? T(-1) : T(1);
-  T gv[3] = {0, 0, 0}, Ec = 0, uc[3] = {0, 0, 0};
+  T gv[3] = {0, 0, 0}, uc[3] = {0, 0, 0};
 #pragma unroll
   for (int Jp = 0; Jp < 8; ++Jp) {
-    const V v = u4[idx[Jp]];
+    V v = Pack4<T>::make(T(0), T(0), T(0), T(0));
+    if (PACKED) {
+      v = u4[idx[Jp]];
+    } else if (idx[Jp] >= 0) {
+      v.x = u[idx[Jp]];
+      v.y = u[idx[Jp] + N];
+      v.z = u[idx[Jp] + 2 * N];
+    }
     if (Jp == 0) {  // J = I: the node itself
       uc[0] = v.x;
       uc[1] = v.y;
       uc[2] = v.z;
     }
-    if (Jp == I) Ec = v.w;  // J = 0: the cell's min corner carries its E
+    if (PACKED && Jp == I) Ec = v.w;
     const T w0 = s0 * v.x, w1 = s1 * v.y, w2 = s2 * v.z;
 #pragma unroll
     for (int r = 0; r < 3; ++r)
@@ -671,7 +699,13 @@ __global__ void __launch_bounds__(128) gs0_cell4_kernel(const int* __restrict__ 
   if (fx) v0 = 0;
   if (fy) v1 = 0;
   if (fz) v2 = 0;
-  u4[g] = Pack4<T>::make(v0, v1, v2, Ec);  // thread 0: the node's own cell
+  if (PACKED) {
+    u4[g] = Pack4<T>::make(v0, v1, v2, Ec);  // thread 0: the node's own cell
+  } else {
+    u[g] = v0;
+    u[g + N] = v1;
+    u[g + 2 * N] = v2;
+  }
 }
 
 // ---------------------------------------------------------------------------

@@ -469,7 +469,7 @@ class Solver {
                 (neg ? -kv[c] : kv[c]) != kc32[(I * 8 + J) * 9 + v * 3 + w] ||
                 (neg ? -kv64[c] : kv64[c]) != kc64[(I * 8 + J) * 9 + v * 3 + w])
               throw CudaError("element table classes are inconsistent", SGS_ERR_INTERNAL);
-            // the reflection symmetry gs0_cell4_kernel relies on: K(I, J) = S K(0, I^J) S
+            // the reflection symmetry gs0_cell_kernel relies on: K(I, J) = S K(0, I^J) S
             const double sg = ((I >> (2 - v)) & 1 ? -1.0 : 1.0) * ((I >> (2 - w)) & 1 ? -1.0 : 1.0);
             if (Kmu[I][J][v][w] != sg * Kmu[0][I ^ J][v][w] || Kla[I][J][v][w] != sg * Kla[0][I ^ J][v][w])
               throw CudaError("element table lacks the reflection symmetry", SGS_ERR_INTERNAL);
@@ -1190,9 +1190,13 @@ class Solver {
         const int c = (boundary ? 8 : 0) + (forward ? k : 7 - k);
         const int lo = d.gs_off[c], cnt = d.gs_off[c + 1] - lo;
         if (cnt == 0) continue;
-        if (!u && boundary) {  // boundary band: few nodes, eight threads per node
-          launch(gs0_cell4_kernel<T>, blocks_for(long(cnt) * 8, 128), 128, 0, d.gs_list.p + lo, cnt, d.nbrz.p, d.u4.p,
-                 b, d.flags.p, int(d.N), T(P.dx));
+        if (cnt <= GS_CELL_NODES) {  // few nodes: eight threads per node
+          if (!u)
+            launch(gs0_cell_kernel<T, true>, blocks_for(long(cnt) * 8, 128), 128, 0, d.gs_list.p + lo, cnt, d.nbrz.p,
+                   d.u4.p, nullptr, nullptr, b, d.flags.p, int(d.N), T(P.dx));
+          else
+            launch(gs0_cell_kernel<T, false>, blocks_for(long(cnt) * 8, 128), 128, 0, d.gs_list.p + lo, cnt, d.nbr.p,
+                   nullptr, u, Edev<T>(), b, d.flags.p, int(d.N), T(P.dx));
           ++launch_counter;
           continue;
         }
