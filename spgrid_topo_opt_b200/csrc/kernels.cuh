@@ -857,7 +857,7 @@ template <typename T>
 __global__ void __launch_bounds__(128) restrict_kernel(int nb, const int* __restrict__ coords,
                                                        const uint32_t* __restrict__ cflags, GridView fine,
                                                        const T* __restrict__ fin, long Nf, T* __restrict__ cout,
-                                                       long Nc) {
+                                                       long Nc, T* __restrict__ zero) {
   constexpr int RX = 9, RY = 9, RZ = 17, RN = RX * RY * RZ;
   __shared__ T sf[3][RN];
   __shared__ int sblk[27];
@@ -903,6 +903,7 @@ __global__ void __launch_bounds__(128) restrict_kernel(int nb, const int* __rest
   cout[t] = (fl & DIR_X) ? T(0) : v0;
   cout[t + Nc] = (fl & DIR_Y) ? T(0) : v1;
   cout[t + 2 * Nc] = (fl & DIR_Z) ? T(0) : v2;
+  if (zero) zero[t] = zero[t + Nc] = zero[t + 2 * Nc] = T(0);  // the coarse iterate starts from zero
 }
 
 // The 3x3x5 coarse nodes that the 4x4x8 fine nodes of a fine block interpolate
@@ -928,7 +929,7 @@ template <typename T>
 __global__ void __launch_bounds__(128) prolongate_kernel(int nb, const int* __restrict__ coords,
                                                          const uint32_t* __restrict__ fflags, GridView coarse,
                                                          const T* __restrict__ cin, long Nc, T* __restrict__ fu,
-                                                         long Nf, int round_out) {
+                                                         long Nf, int round_out, int onto_zero) {
   __shared__ T sc[3][45];
   const int bi = blockIdx.x, e = threadIdx.x;
   if (bi >= nb) return;
@@ -937,7 +938,8 @@ __global__ void __launch_bounds__(128) prolongate_kernel(int nb, const int* __re
   stage_coarse_patch<T>(sc, FX, FY, FZ, coarse, cin, Nc);
   const int lx = e >> 5, ly = (e >> 3) & 3, lz = e & 7;
   const long t = long(bi) * 128 + e;
-  T v0 = fu[t], v1 = fu[t + Nf], v2 = fu[t + 2 * Nf];
+  T v0 = 0, v1 = 0, v2 = 0;
+  if (!onto_zero) v0 = fu[t], v1 = fu[t + Nf], v2 = fu[t + 2 * Nf];  // else fu is zero and only written
   for (int q = 0; q < 8; ++q) {
     const int ii = q >> 2, jj = (q >> 1) & 1, kk = q & 1;
     const double wx = (lx & 1) ? 0.5 : (ii ? 0.0 : 1.0);

@@ -536,30 +536,41 @@ __global__ void sgj_mirror_kernel(double* M, long ld) {
 // the level take b, DOF nodes then get the exact solution x = M^-1 b.
 // ---------------------------------------------------------------------------
 template <typename T>
-__global__ void bottom_gather_kernel(int ndof, const int* __restrict__ dof_node, const int* __restrict__ dof_pos,
-                                     const T* __restrict__ b, long N, double* __restrict__ xb) {
+__global__ void bottom_gather_kernel(const int* __restrict__ node_pos, const T* __restrict__ b, long N,
+                                     double* __restrict__ xb, T* __restrict__ u) {
   pdl_wait();
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= ndof) return;
-  long n = dof_node[i];
-  double* x = xb + dof_pos[i];
-  x[0] = double(b[n]);
-  x[1] = double(b[n + N]);
-  x[2] = double(b[n + 2 * N]);
+  const long n = long(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (n >= N) return;
+  const int p = node_pos[n];
+#pragma unroll
+  for (int v = 0; v < 3; ++v) {
+    if (p >= 0) xb[p + v] = double(b[n + v * N]);
+    else u[n + v * N] = b[n + v * N];  // nodes without unknowns keep b
+  }
 }
 
-// y = M x, one warp per row
+// y = M x, one warp per row, written to the level's field: row r is entry
+// out[r] of u (-1: padding)
+template <typename T>
 __global__ void gemv_kernel(const double* __restrict__ M, long ld, long n, const double* __restrict__ x,
-                            double* __restrict__ y) {
-  pdl_wait();
+                            const int* __restrict__ out, T* __restrict__ u) {
   const long row = (long(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
-  if (row >= n) return;
-  const double* m = M + row * ld;
-  double s = 0;
-  for (long c = lane; c < n; c += 32) s += m[c] * x[c];
+  const int to = row < n ? out[row] : -1;
+  pdl_wait();
+  if (to < 0) return;
+  const double2* m = reinterpret_cast<const double2*>(M + row * ld);
+  const double2* v = reinterpret_cast<const double2*>(x);
+  double s0 = 0, s1 = 0;
+#pragma unroll 4
+  for (long c = lane; c < n / 2; c += 32) {
+    const double2 a = __ldcs(m + c), w = v[c];
+    s0 = fma(a.x, w.x, s0);
+    s1 = fma(a.y, w.y, s1);
+  }
+  double s = s0 + s1;
   for (int o = 16; o; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-  if (lane == 0) y[row] = s;
+  if (lane == 0) u[to] = T(s);
 }
 
 // y = M x with an FP32 copy of M (ld a multiple of 128, rows 16-byte aligned),
@@ -568,7 +579,8 @@ __global__ void gemv_kernel(const double* __restrict__ M, long ld, long n, const
 // FP32 right-hand side), so the loop streams only M.
 constexpr int GEMV32_ROWS = 32;
 __global__ void __launch_bounds__(1024) gemv32_kernel(const float* __restrict__ M, long ld, long n,
-                                                      const double* __restrict__ x, double* __restrict__ y) {
+                                                      const double* __restrict__ x, const int* __restrict__ out,
+                                                      float* __restrict__ u) {
   extern __shared__ float4 xs4[];
   float* xs = reinterpret_cast<float*>(xs4);
   pdl_wait();
@@ -589,20 +601,7 @@ __global__ void __launch_bounds__(1024) gemv32_kernel(const float* __restrict__ 
   }
   double s = double(s0) + double(s1);
   for (int o = 16; o; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-  if (lane == 0) y[row] = s;
-}
-
-template <typename T>
-__global__ void bottom_scatter_kernel(int ndof, const int* __restrict__ dof_node, const int* __restrict__ dof_pos,
-                                      const double* __restrict__ xs, T* __restrict__ u, long N) {
-  pdl_wait();
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= ndof) return;
-  long n = dof_node[i];
-  const double* x = xs + dof_pos[i];
-  u[n] = T(x[0]);
-  u[n + N] = T(x[1]);
-  u[n + 2 * N] = T(x[2]);
+  if (lane == 0 && out[row] >= 0) u[out[row]] = float(s);
 }
 
 }  // namespace sgs

@@ -101,11 +101,12 @@ struct Level {
 struct Bottom {
   int ndof_nodes = 0;
   long n = 0, ld = 0;
-  DevBuf<int> dof_node, dof_pos, node_pos;  // nodes with unknowns, their first unknowns, and those by node
+  DevBuf<int> dof_node, node_pos;  // nodes with unknowns; first unknown by node (-1: none)
+  DevBuf<int> row_out;             // unknown -> entry of the level's field (-1: padding)
   BottomOrder order;
   std::vector<int32_t> ordered_nodes;  // the nodes `order` was made for
   DevBuf<int> tiles, pad;              // BottomOrder::list and pad on the device
-  DevBuf<double> Minv, xb, xs;
+  DevBuf<double> Minv, xb;
   DevBuf<float> Minv32;  // mixed precision: the FP32 V-cycle applies an FP32 copy of Minv
 };
 
@@ -294,6 +295,7 @@ class Solver {
   DevBuf<int> load_node;     // loaded nodes, once each (the compliance f.u)
   DevBuf<double> load_val;
   DevBuf<double> red;      // reduction partials
+  DevBuf<unsigned> ticket;  // arrivals of a reducing kernel's CTAs (zero between kernels)
   DevBuf<double> scal;     // device scalars: 0 rho, 1 rho_old, 2 sq, 3 norm, 4 beta, 5 alpha, 6 -alpha, 7 breakdown
   double* h_scal = nullptr;  // pinned mirror
   // input block map for packing
@@ -963,7 +965,10 @@ class Solver {
       std::vector<int32_t> node_pos(size_t(d.N), -1);
       for (size_t k = 0; k < dof_node.size(); ++k) node_pos[size_t(dof_node[k])] = o.pos[k];
       bottom.dof_node.upload(dof_node, stream);
-      bottom.dof_pos.upload(o.pos, stream);
+      std::vector<int32_t> row_out(size_t(o.ld), -1);
+      for (size_t k = 0; k < dof_node.size(); ++k)
+        for (int v = 0; v < 3; ++v) row_out[size_t(o.pos[k] + v)] = dof_node[k] + v * int(d.N);
+      bottom.row_out.upload(row_out, stream);
       bottom.node_pos.upload(node_pos, stream);
       bottom.tiles.upload(o.list, stream);
       bottom.pad.upload(o.pad, stream);
@@ -972,9 +977,7 @@ class Solver {
     }
     bottom.ld = bottom.order.ld;
     bottom.xb.alloc(size_t(bottom.ld));
-    bottom.xs.alloc(size_t(bottom.ld));
     bottom.xb.zero(stream);
-    bottom.xs.zero(stream);
     if (bottom.n == 0) return;
     bottom.Minv.alloc(size_t(bottom.ld) * bottom.ld);
     bottom.Minv.zero(stream);
@@ -1114,6 +1117,8 @@ class Solver {
     red.alloc(size_t(std::max<long>(2048, P.levels[0].nb)));  // reduction partials (one per level-0 block at most)
     scal.alloc(16);
     scal.zero(stream);
+    ticket.alloc(1);
+    ticket.zero(stream);
     in_block.upload(P.in_block, stream);
     in_zoff.upload(P.in_zoff, stream);
     out_disp.alloc(P.in_block.size() * 64 * 4);
@@ -1249,17 +1254,17 @@ class Solver {
   }
 
   template <typename T>
-  void restrict_to(int lc, const T* fine_field) {
+  void restrict_to(int lc, const T* fine_field, T* zero = nullptr) {
     Level<T>& c = lev<T>(lc);
     Level<T>& fl = lev<T>(lc - 1);
     if (c.N == 0) return;
     launch(restrict_kernel<T>, blocks_for(c.N, 128), 128, 0, c.nb, c.coords.p, c.flags.p, fl.grid, fine_field, fl.N,
-                                                                c.b.p, c.N);
+                                                                c.b.p, c.N, zero);
     ++launch_counter;
   }
 
   template <typename T>
-  void prolongate_to(int lf, T* fine_u, int round = -1) {
+  void prolongate_to(int lf, T* fine_u, int round = -1, bool onto_zero = false) {
     Level<T>& fl = lev<T>(lf);
     Level<T>& c = lev<T>(lf + 1);
     if (fl.N == 0) return;
@@ -1270,7 +1275,7 @@ class Solver {
       return;
     }
     launch(prolongate_kernel<T>, blocks_for(fl.N, 128), 128, 0, fl.nb, fl.coords.p, fl.flags.p, c.grid, c.u.p, c.N,
-                                                                   fine_u, fl.N, round < 0 ? (round_ref() ? 1 : 0) : round);
+                                                                   fine_u, fl.N, round < 0 ? (round_ref() ? 1 : 0) : round, onto_zero ? 1 : 0);
     ++launch_counter;
   }
 
@@ -1290,21 +1295,17 @@ class Solver {
   void bottom_dense(int l, bool round) {
     Level<T>& d = lev<T>(l);
     // nodes without unknowns keep b (the reference copies b in and out)
-    SGS_CUDA(cudaMemcpyAsync(d.u.p, d.b.p, 3 * d.N * sizeof(T), cudaMemcpyDeviceToDevice, stream));
+    launch(bottom_gather_kernel<T>, blocks_for(d.N, 256), 256, 0, bottom.node_pos.p, d.b.p, d.N, bottom.xb.p, d.u.p);
+    ++launch_counter;
     if (bottom.ndof_nodes > 0) {
-      launch(bottom_gather_kernel<T>, blocks_for(bottom.ndof_nodes, 128), 128, 0, bottom.ndof_nodes, bottom.dof_node.p,
-             bottom.dof_pos.p,
-                                                                                     d.b.p, d.N, bottom.xb.p);
-      if (sizeof(T) == 4 && bottom.Minv32.p)  // the FP32 V-cycle applies the FP32 copy
+      if constexpr (sizeof(T) == 4) {  // the FP32 V-cycle applies the FP32 copy
         launch(gemv32_kernel, blocks_for(bottom.ld, GEMV32_ROWS), 1024, size_t(bottom.ld) * sizeof(float),
-               bottom.Minv32.p, bottom.ld, bottom.ld, bottom.xb.p, bottom.xs.p);
-      else
-        launch(gemv_kernel, blocks_for(bottom.ld * 32, 256), 256, 0, bottom.Minv.p, bottom.ld, bottom.ld, bottom.xb.p,
-               bottom.xs.p);
-      launch(bottom_scatter_kernel<T>, blocks_for(bottom.ndof_nodes, 128), 128, 0, bottom.ndof_nodes,
-                                                                                      bottom.dof_node.p, bottom.dof_pos.p, bottom.xs.p,
-                                                                                      d.u.p, d.N);
-      launch_counter += 3;
+               bottom.Minv32.p, bottom.ld, bottom.ld, bottom.xb.p, bottom.row_out.p, d.u.p);
+      } else {
+        launch(gemv_kernel<T>, blocks_for(bottom.ld * 32, 256), 256, 0, bottom.Minv.p, bottom.ld, bottom.ld, bottom.xb.p,
+               bottom.row_out.p, d.u.p);
+      }
+      ++launch_counter;
     }
     if (round) round3(d, d.u.p);
   }
@@ -1338,10 +1339,8 @@ class Solver {
       Level<double>& d = *L64[l];
       inner_sweeps(l, true);
       Level<double>& c = *L64[l + 1];
-      SGS_CUDA(cudaMemsetAsync(c.u.p, 0, 3 * c.N * sizeof(double), stream));
-      SGS_CUDA(cudaMemsetAsync(c.b.p, 0, 3 * c.N * sizeof(double), stream));
       stencil<double, SOP_RES>(l, nullptr, d.nb, d.u.p, nullptr, d.b.p, d.r.p, 0);
-      restrict_to<double>(l + 1, d.r.p);
+      restrict_to<double>(l + 1, d.r.p, c.u.p);
     }
     bottom_dense<double>(n - 1, false);
     for (int l = n - 2; l >= top; --l) {
@@ -1405,7 +1404,7 @@ class Solver {
 
   // V-cycle (Run_VCycle): level-0 right-hand side b0, correction written to u0.
   template <typename T>
-  void vcycle(const T* b0, T* u0) {
+  void vcycle(const T* b0, T* u0, bool reset = true) {
     const int n = nout();
     const int ex = P.explicit_level;
     const bool rr = round_ref();
@@ -1413,8 +1412,10 @@ class Solver {
     // u0 == nullptr: the packed level-0 iterate l0.u4
     const bool packed = u0 == nullptr;
     if (packed) {
-      launch(reset_u4_kernel<T>, blocks_for(l0.N, 256), 256, 0, l0.u4.p, Edev<T>(), l0.N);
-      ++launch_counter;
+      if (reset) {
+        launch(reset_u4_kernel<T>, blocks_for(l0.N, 256), 256, 0, l0.u4.p, Edev<T>(), l0.N);
+        ++launch_counter;
+      }
     } else {
       SGS_CUDA(cudaMemsetAsync(u0, 0, 3 * l0.N * sizeof(T), stream));
     }
@@ -1430,9 +1431,9 @@ class Solver {
     for (int l = 0; l < n - 1; ++l) {
       const bool smooth = l == 0 || l >= ex;
       if (smooth) sweeps<T>(l, U(l), B(l), true);
-      Level<T>& c = lev<T>(l + 1);
-      SGS_CUDA(cudaMemsetAsync(c.u.p, 0, 3 * c.N * sizeof(T), stream));
-      SGS_CUDA(cudaMemsetAsync(c.b.p, 0, 3 * c.N * sizeof(T), stream));
+      // the next level's iterate starts from zero: where it is smoothed the
+      // restriction clears it, elsewhere it is only written
+      T* zero = l + 1 < n - 1 && l + 1 >= ex ? lev<T>(l + 1).u.p : nullptr;
       Level<T>& d = lev<T>(l);
       if (smooth) {
         if (l == 0) {
@@ -1445,14 +1446,14 @@ class Solver {
         } else {
           stencil<T, SOP_RES>(l, nullptr, d.nb, U(l), nullptr, B(l), d.r.p, rr ? 1 : 0);
         }
-        restrict_to<T>(l + 1, d.r.p);
+        restrict_to<T>(l + 1, d.r.p, zero);
       } else {
-        restrict_to<T>(l + 1, B(l));
+        restrict_to<T>(l + 1, B(l), zero);
       }
     }
     bottom_solve<T>(n - 1);
     for (int l = n - 2; l >= 0; --l) {
-      prolongate_to<T>(l, U(l));
+      prolongate_to<T>(l, U(l), -1, l > 0 && l < ex);
       if (l == 0 || l >= ex) sweeps<T>(l, U(l), B(l), false);
     }
   }
@@ -1471,7 +1472,7 @@ class Solver {
   void axpy(double* dst, double sign, int coef_slot, const double* xv, const double* yv);
   int precondition();  // returns the number of rho partials it wrote
   void stage_residual();
-  void record_iteration();
+  void record_iteration(bool norm);  // norm: reduce |r|_inf too (else the caller's next kernel does)
   void solve();
   // displacements [nblocks][64][4] to host memory, records `pitch` bytes apart (0: packed)
   void pack_outputs(void* disp, size_t pitch = 0);
@@ -1581,11 +1582,12 @@ __global__ void linf_partial_kernel(const double* __restrict__ a, long n, double
   }
 }
 
-// Fixed-order final reduction by one CTA of FIN_THREADS; op 0 = sum, 1 = max.
+// Fixed-order final reduction by one CTA of FIN_THREADS (the matvec leaves a
+// partial per CTA, 170357 at 1024^3: 24 us with 256 threads); op 0 = sum, 1 = max.
 // Also derives the PCG scalars: what = 0: rho -> beta = rho/rho_old;
 // what = 1: sq -> alpha, -alpha, breakdown flag; what = 2: norm; what = 4: norm
 // and rho_old = rho (the end of an iteration).
-constexpr int FIN_THREADS = 256;
+constexpr int FIN_THREADS = 1024;
 __global__ void finish_reduce_kernel(const double* __restrict__ part, int np, int op, double* scal, int what) {
   pdl_wait();
   __shared__ double sm[FIN_THREADS];
@@ -1675,80 +1677,22 @@ __global__ void precond_out4_kernel(const typename Pack4<T>::type* __restrict__ 
   }
 }
 
-// End of a PCG iteration (CONJUGATE_GRADIENT.cpp:54-57, 32-33): x += alpha s,
-// r -= alpha q (float-rounded like CG_VECTOR in the reference mode), then
-// Project_Nullspace(r), per-CTA partials of |r|_inf and, when b32 is given, the
-// single-precision copy of r that the next V-cycle starts from.
-__global__ void cg_update_kernel(double* x, const double* __restrict__ s, double* f, const double* __restrict__ q,
-                                 const double* __restrict__ scal, const uint32_t* __restrict__ flags, long N,
-                                 int float_round, float* __restrict__ b32, double* __restrict__ part) {
-  pdl_wait();
-  __shared__ double sm[RED_THREADS / 32];
-  const double a = scal[5], na = scal[6];
-  double m = 0;
-  for (long i = long(blockIdx.x) * blockDim.x + threadIdx.x; i < N; i += long(gridDim.x) * blockDim.x) {
-    const bool act = flags[i] & ACTIVE_NODE;
-#pragma unroll
-    for (int v = 0; v < 3; ++v) {
-      const long k = i + v * N;
-      double xv, fv;
-      if (float_round) {
-        xv = double(__fadd_rn(__fmul_rn(float(a), float(s[k])), float(x[k])));
-        fv = double(__fadd_rn(__fmul_rn(float(na), float(q[k])), float(f[k])));
-      } else {
-        xv = a * s[k] + x[k];
-        fv = na * q[k] + f[k];
-      }
-      if (!act) fv = 0;
-      x[k] = xv;
-      f[k] = fv;
-      if (b32) b32[k] = float(fv);
-      m = fmax(m, fabs(fv));
-    }
-  }
-  for (int o = 16; o; o >>= 1) m = fmax(m, __shfl_down_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = m;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = 0;
-    for (int w = 0; w < RED_THREADS / 32; ++w) t = fmax(t, sm[w]);
-    part[blockIdx.x] = t;
-  }
-}
+// The pair kernels of a PCG iteration work on two nodes per thread with 16-byte
+// loads and stores (N is a multiple of 128) and skip pairs of inactive nodes:
+// there every PCG vector is zero for the whole solve (Project_Nullspace zeroes
+// them, K u vanishes where no active cell touches a node, x starts at zero), so
+// only the flags are read for them and the sectors that hold no active node are
+// never fetched.  They are bound by HBM; what they move per iteration and active
+// node is 44 + 116 + 88 B (mixed) and 3 vectors less than as separate steps: z
+// stays in the packed iterate (never written out as a planar vector), x is
+// updated together with the search direction, which reads s anyway, and the
+// packed iterate is cleared for the next V-cycle by the kernel that reads it last.
 
-// precond_out4_kernel over node pairs: two nodes per thread with 16-byte loads and
-// stores (N is a multiple of 128), the same arithmetic per node.  The pair
-// kernels skip pairs of inactive nodes: there every PCG vector is zero for the
-// whole solve (Project_Nullspace zeroes them, K u vanishes where no active cell
-// touches a node, x starts at zero), so only the flags are read for them and
-// the sectors that hold no active node are never fetched.
-template <typename T>
-__global__ void __launch_bounds__(RED_THREADS, 4) precond_out4_pair_kernel(const typename Pack4<T>::type* __restrict__ z4,
-                                                                       double* __restrict__ q,
-                                                                       const double* __restrict__ f,
-                                                                       const uint32_t* __restrict__ flags, long N,
-                                                                       double* __restrict__ part) {
-  pdl_wait();
+// per-CTA partials in part; the CTA that finishes last sums them in index order
+// (fixed whatever the order of arrival): rho, beta
+__device__ void finish_rho(double s, double* part, double* scal, unsigned* ticket) {
   __shared__ double sm[RED_THREADS / 32];
-  double s = 0;
-  const long P = N >> 1;
-  for (long p = long(blockIdx.x) * blockDim.x + threadIdx.x; p < P; p += long(gridDim.x) * blockDim.x) {
-    const uint2 fl = reinterpret_cast<const uint2*>(flags)[p];
-    if (!((fl.x | fl.y) & ACTIVE_NODE)) continue;
-    const auto za = z4[2 * p], zb = z4[2 * p + 1];
-    const double zc[2][3] = {{double(za.x), double(za.y), double(za.z)}, {double(zb.x), double(zb.y), double(zb.z)}};
-    const uint32_t fls[2] = {fl.x, fl.y};
-#pragma unroll
-    for (int v = 0; v < 3; ++v) {
-      double2 out;
-      const double2 fv = reinterpret_cast<const double2*>(f + v * N)[p];
-      out.x = ((fls[0] & ACTIVE_NODE) && !(fls[0] & (DIR_X << v))) ? zc[0][v] : 0.0;
-      out.y = ((fls[1] & ACTIVE_NODE) && !(fls[1] & (DIR_X << v))) ? zc[1][v] : 0.0;
-      reinterpret_cast<double2*>(q + v * N)[p] = out;
-      s += out.x * fv.x;
-      s += out.y * fv.y;
-    }
-  }
+  __shared__ bool last;
   for (int o = 16; o; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
   if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = s;
   __syncthreads();
@@ -1756,19 +1700,128 @@ __global__ void __launch_bounds__(RED_THREADS, 4) precond_out4_pair_kernel(const
     double t = 0;
     for (int w = 0; w < RED_THREADS / 32; ++w) t += sm[w];
     part[blockIdx.x] = t;
+    __threadfence();
+    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  double t = 0;
+  for (int i = threadIdx.x; i < int(gridDim.x); i += RED_THREADS) t += __ldcg(part + i);
+  for (int o = 16; o; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = t;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    t = 0;
+    for (int w = 0; w < RED_THREADS / 32; ++w) t += sm[w];
+    scal[0] = t;            // rho
+    scal[4] = t / scal[1];  // beta = rho / rho_old
+    *ticket = 0;
   }
 }
 
-// cg_update_kernel over node pairs (16-byte loads and stores), the same arithmetic per node.
-__global__ void __launch_bounds__(RED_THREADS, 4) cg_update_pair_kernel(double* __restrict__ x, const double* __restrict__ s,
-                                                                    double* __restrict__ f, const double* __restrict__ q,
-                                                                    const double* __restrict__ scal,
-                                                                    const uint32_t* __restrict__ flags, long N,
-                                                                    int float_round, float* __restrict__ b32,
-                                                                    double* __restrict__ part) {
+// rho = z.r with z projected (Project, Project_Nullspace; KRYLOV_SYSTEM_BASE.cpp:25-31)
+template <typename T>
+__global__ void __launch_bounds__(RED_THREADS, 4) rho_pair_kernel(const typename Pack4<T>::type* __restrict__ z4,
+                                                                  const double* __restrict__ f,
+                                                                  const uint32_t* __restrict__ flags, long N,
+                                                                  double* part, double* scal, unsigned* ticket) {
+  pdl_wait();
+  double s = 0;
+  const long P = N >> 1;
+  for (long p = long(blockIdx.x) * blockDim.x + threadIdx.x; p < P; p += long(gridDim.x) * blockDim.x) {
+    const uint2 fl = reinterpret_cast<const uint2*>(flags)[p];
+    if (!((fl.x | fl.y) & ACTIVE_NODE)) continue;
+    const auto za = z4[2 * p], zb = z4[2 * p + 1];
+    const double zc[2][3] = {{double(za.x), double(za.y), double(za.z)}, {double(zb.x), double(zb.y), double(zb.z)}};
+#pragma unroll
+    for (int v = 0; v < 3; ++v) {
+      const double2 fv = reinterpret_cast<const double2*>(f + v * N)[p];
+      s += (((fl.x & ACTIVE_NODE) && !(fl.x & (DIR_X << v))) ? zc[0][v] : 0.0) * fv.x;
+      s += (((fl.y & ACTIVE_NODE) && !(fl.y & (DIR_X << v))) ? zc[1][v] : 0.0) * fv.y;
+    }
+  }
+  finish_rho(s, part, scal, ticket);
+}
+
+// x += alpha s (the last iteration's step), then s = beta s + z
+// (CONJUGATE_GRADIENT.cpp:44-54).  PACKED: z from the V-cycle's packed iterate,
+// projected, which is left at zero for the next V-cycle; else z = q.
+template <typename T, bool PACKED>
+__global__ void __launch_bounds__(RED_THREADS, 4) direction_pair_kernel(double* __restrict__ x, double* __restrict__ s,
+                                                                        typename Pack4<T>::type* __restrict__ z4,
+                                                                        const double* __restrict__ q,
+                                                                        const double* __restrict__ scal, long N,
+                                                                        int float_round,
+                                                                        const uint32_t* __restrict__ flags) {
+  pdl_wait();
+  const double beta = scal[4], alpha = scal[5];
+  const long P = N >> 1;
+  for (long p = long(blockIdx.x) * blockDim.x + threadIdx.x; p < P; p += long(gridDim.x) * blockDim.x) {
+    const uint2 fl = reinterpret_cast<const uint2*>(flags)[p];
+    if (!((fl.x | fl.y) & ACTIVE_NODE)) continue;
+    double zc[2][3];
+    if (PACKED) {
+      auto za = z4[2 * p], zb = z4[2 * p + 1];
+      zc[0][0] = za.x, zc[0][1] = za.y, zc[0][2] = za.z;
+      zc[1][0] = zb.x, zc[1][1] = zb.y, zc[1][2] = zb.z;
+      za.x = za.y = za.z = zb.x = zb.y = zb.z = T(0);
+      z4[2 * p] = za;
+      z4[2 * p + 1] = zb;
+#pragma unroll
+      for (int v = 0; v < 3; ++v) {
+        if (!(fl.x & ACTIVE_NODE) || (fl.x & (DIR_X << v))) zc[0][v] = 0;
+        if (!(fl.y & ACTIVE_NODE) || (fl.y & (DIR_X << v))) zc[1][v] = 0;
+      }
+    }
+#pragma unroll
+    for (int v = 0; v < 3; ++v) {
+      const long o = v * P + p;
+      const double2 a = reinterpret_cast<const double2*>(s)[o], xv = reinterpret_cast<const double2*>(x)[o];
+      const double2 z = PACKED ? make_double2(zc[0][v], zc[1][v]) : reinterpret_cast<const double2*>(q)[o];
+      double2 r, xo;
+      if (float_round) {
+        xo.x = double(__fadd_rn(__fmul_rn(float(alpha), float(a.x)), float(xv.x)));
+        xo.y = double(__fadd_rn(__fmul_rn(float(alpha), float(a.y)), float(xv.y)));
+        r.x = double(__fadd_rn(__fmul_rn(float(beta), float(a.x)), float(z.x)));
+        r.y = double(__fadd_rn(__fmul_rn(float(beta), float(a.y)), float(z.y)));
+      } else {
+        xo.x = alpha * a.x + xv.x;
+        xo.y = alpha * a.y + xv.y;
+        r.x = beta * a.x + z.x;
+        r.y = beta * a.y + z.y;
+      }
+      reinterpret_cast<double2*>(x)[o] = xo;
+      reinterpret_cast<double2*>(s)[o] = r;
+    }
+  }
+}
+
+// x += alpha s of the last iteration, then x += u0 (the lifted start)
+__global__ void finish_solution_kernel(double* __restrict__ x, const double* __restrict__ s,
+                                       const double* __restrict__ u0, const double* __restrict__ scal, long n,
+                                       int float_round) {
+  pdl_wait();
+  const long i = long(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const double a = scal[5];
+  const double xv = float_round ? double(__fadd_rn(__fmul_rn(float(a), float(s[i])), float(x[i]))) : a * s[i] + x[i];
+  x[i] = xv + u0[i];
+}
+
+// End of a PCG iteration (CONJUGATE_GRADIENT.cpp:54-57, 32-33) over node pairs:
+// r -= alpha q (float-rounded like CG_VECTOR in the reference mode), then
+// Project_Nullspace(r), per-CTA partials of |r|_inf and, when b32 is given, the
+// single-precision copy of r that the next V-cycle starts from.
+__global__ void __launch_bounds__(RED_THREADS, 4) residual_pair_kernel(double* __restrict__ f, const double* __restrict__ q,
+                                                                       const double* __restrict__ scal,
+                                                                       const uint32_t* __restrict__ flags, long N,
+                                                                       int float_round, float* __restrict__ b32,
+                                                                       double* __restrict__ part) {
   pdl_wait();
   __shared__ double sm[RED_THREADS / 32];
-  const double a = scal[5], na = scal[6];
+  const double na = scal[6];
   double m = 0;
   const long P = N >> 1;
   for (long p = long(blockIdx.x) * blockDim.x + threadIdx.x; p < P; p += long(gridDim.x) * blockDim.x) {
@@ -1778,23 +1831,17 @@ __global__ void __launch_bounds__(RED_THREADS, 4) cg_update_pair_kernel(double* 
 #pragma unroll
     for (int v = 0; v < 3; ++v) {
       const long o = v * (N >> 1) + p;
-      const double2 xv = reinterpret_cast<const double2*>(x)[o], sv = reinterpret_cast<const double2*>(s)[o];
       const double2 fv = reinterpret_cast<const double2*>(f)[o], qv = reinterpret_cast<const double2*>(q)[o];
-      double2 xo, fo;
+      double2 fo;
       if (float_round) {
-        xo.x = double(__fadd_rn(__fmul_rn(float(a), float(sv.x)), float(xv.x)));
-        xo.y = double(__fadd_rn(__fmul_rn(float(a), float(sv.y)), float(xv.y)));
         fo.x = double(__fadd_rn(__fmul_rn(float(na), float(qv.x)), float(fv.x)));
         fo.y = double(__fadd_rn(__fmul_rn(float(na), float(qv.y)), float(fv.y)));
       } else {
-        xo.x = a * sv.x + xv.x;
-        xo.y = a * sv.y + xv.y;
         fo.x = na * qv.x + fv.x;
         fo.y = na * qv.y + fv.y;
       }
       if (!act[0]) fo.x = 0;
       if (!act[1]) fo.y = 0;
-      reinterpret_cast<double2*>(x)[o] = xo;
       reinterpret_cast<double2*>(f)[o] = fo;
       if (b32) reinterpret_cast<float2*>(b32)[o] = make_float2(float(fo.x), float(fo.y));
       m = fmax(m, fmax(fabs(fo.x), fabs(fo.y)));
@@ -1807,35 +1854,6 @@ __global__ void __launch_bounds__(RED_THREADS, 4) cg_update_pair_kernel(double* 
     double t = 0;
     for (int w = 0; w < RED_THREADS / 32; ++w) t = fmax(t, sm[w]);
     part[blockIdx.x] = t;
-  }
-}
-
-// dst = c*x + y over node pairs of three-component fields [3][N] (16-byte loads
-// and stores), grid-stride; pairs of inactive nodes are skipped (both operands
-// are zero there)
-__global__ void __launch_bounds__(RED_THREADS, 4) axpy_pair_kernel(double* dst, const double* __restrict__ scal, int slot,
-                                                               const double* xv, const double* yv, long N,
-                                                               int float_round, const uint32_t* __restrict__ flags) {
-  pdl_wait();
-  const double c = scal[slot];
-  const long P = N >> 1;
-  for (long p = long(blockIdx.x) * blockDim.x + threadIdx.x; p < P; p += long(gridDim.x) * blockDim.x) {
-    const uint2 fl = reinterpret_cast<const uint2*>(flags)[p];
-    if (!((fl.x | fl.y) & ACTIVE_NODE)) continue;
-#pragma unroll
-    for (int v = 0; v < 3; ++v) {
-      const long o = v * P + p;
-      const double2 a = reinterpret_cast<const double2*>(xv)[o], b = reinterpret_cast<const double2*>(yv)[o];
-      double2 r;
-      if (float_round) {
-        r.x = double(__fadd_rn(__fmul_rn(float(c), float(a.x)), float(b.x)));
-        r.y = double(__fadd_rn(__fmul_rn(float(c), float(a.y)), float(b.y)));
-      } else {
-        r.x = c * a.x + b.x;
-        r.y = c * a.y + b.y;
-      }
-      reinterpret_cast<double2*>(dst)[o] = r;
-    }
   }
 }
 
@@ -1875,12 +1893,6 @@ __global__ void scatter_force_kernel(double* s, const int* __restrict__ node, co
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   for (int v = 0; v < 3; ++v) s[node[i] + v * N] = val[3 * i + v];
-}
-
-__global__ void add_kernel(double* a, const double* __restrict__ b, long n) {
-  pdl_wait();
-  long i = long(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i < n) a[i] += b[i];
 }
 
 // Output packing (SPGrid_CPU_Solver.cpp:343-364): per input block node
@@ -2057,16 +2069,14 @@ int Solver::precondition() {
     Level<float>& m0 = *L32[0];
     if (packed0()) {
       vcycle<float>(m0.b.p, nullptr);
-      launch(precond_out4_pair_kernel<float>, PAIR_BLOCKS, RED_THREADS, 0, m0.u4.p, q.p, f.p, l0.flags.p, N, red.p);
-      parts = PAIR_BLOCKS;
+      launch(precond_out4_kernel<float>, RED_BLOCKS, RED_THREADS, 0, m0.u4.p, q.p, f.p, l0.flags.p, N, red.p);
     } else {
       vcycle<float>(m0.b.p, m0.u.p);
       launch(precond_out_kernel<float>, RED_BLOCKS, RED_THREADS, 0, m0.u.p, q.p, f.p, l0.flags.p, N, red.p);
     }
   } else if (packed0()) {
     vcycle<double>(f.p, nullptr);
-    launch(precond_out4_pair_kernel<double>, PAIR_BLOCKS, RED_THREADS, 0, l0.u4.p, q.p, f.p, l0.flags.p, N, red.p);
-    parts = PAIR_BLOCKS;
+    launch(precond_out4_kernel<double>, RED_BLOCKS, RED_THREADS, 0, l0.u4.p, q.p, f.p, l0.flags.p, N, red.p);
   } else {
     vcycle<double>(f.p, q.p);
     launch(precond_out_kernel<double>, RED_BLOCKS, RED_THREADS, 0, q.p, q.p, f.p, l0.flags.p, N, red.p);
@@ -2138,19 +2148,42 @@ void Solver::stage_residual() {
 }
 
 // One PCG iteration after the convergence test (CONJUGATE_GRADIENT.cpp:41-57) plus
-// the next iteration's Project_Nullspace and norm (:32-33).
-void Solver::record_iteration() {
+// the next iteration's Project_Nullspace and norm (:32-33).  The step x += alpha s
+// is taken by the next iteration's direction_pair_kernel, or after the loop.
+void Solver::record_iteration(bool norm) {
   Level<double>& l0 = *L64[0];
-  const int parts = precondition();                                      // q = z, rho partials
-  launch(finish_reduce_kernel, 1, FIN_THREADS, 0, red.p, parts, 0, scal.p, 0);  // rho, beta
-  launch(axpy_pair_kernel, PAIR_BLOCKS, RED_THREADS, 0, s.p, scal.p, 4, s.p, q.p, N0(),
-         round_ref() ? 1 : 0, l0.flags.p);                               // s = beta*s + z
+  const int fr = round_ref() ? 1 : 0;
+  if (packed0() && !P.disable_mg) {  // z stays in the packed iterate
+    if (mixed()) {
+      Level<float>& m0 = *L32[0];
+      vcycle<float>(m0.b.p, nullptr, false);
+      launch(rho_pair_kernel<float>, PAIR_BLOCKS, RED_THREADS, 0, m0.u4.p, f.p, l0.flags.p, l0.N, red.p, scal.p,
+             ticket.p);
+      launch(direction_pair_kernel<float, true>, PAIR_BLOCKS, RED_THREADS, 0, x.p, s.p, m0.u4.p, nullptr, scal.p, l0.N,
+             0, l0.flags.p);
+    } else {
+      vcycle<double>(f.p, nullptr, false);
+      launch(rho_pair_kernel<double>, PAIR_BLOCKS, RED_THREADS, 0, l0.u4.p, f.p, l0.flags.p, l0.N, red.p, scal.p,
+             ticket.p);
+      launch(direction_pair_kernel<double, true>, PAIR_BLOCKS, RED_THREADS, 0, x.p, s.p, l0.u4.p, nullptr, scal.p, l0.N,
+             0, l0.flags.p);
+    }
+    launch_counter += 2;
+  } else {
+    const int parts = precondition();                                    // q = z, rho partials
+    launch(finish_reduce_kernel, 1, FIN_THREADS, 0, red.p, parts, 0, scal.p, 0);  // rho, beta
+    launch(direction_pair_kernel<double, false>, PAIR_BLOCKS, RED_THREADS, 0, x.p, s.p, nullptr, q.p, scal.p, l0.N, fr,
+           l0.flags.p);
+    launch_counter += 2;
+  }
   level0<double, OP_KUP>(s.p, nullptr, q.p);                             // q = K s, Project, s.q partials
   launch(finish_reduce_kernel, 1, FIN_THREADS, 0, red.p, int(modal_grid(l0.nb)), 0, scal.p, 1);  // alpha
-  launch(cg_update_pair_kernel, PAIR_BLOCKS, RED_THREADS, 0, x.p, s.p, f.p, q.p, scal.p, l0.flags.p, l0.N,
-         round_ref() ? 1 : 0, (mixed() && !P.disable_mg) ? L32[0]->b.p : (float*)nullptr, red.p);
+  launch(residual_pair_kernel, PAIR_BLOCKS, RED_THREADS, 0, f.p, q.p, scal.p, l0.flags.p, l0.N, fr,
+         (mixed() && !P.disable_mg) ? L32[0]->b.p : (float*)nullptr, red.p);
+  launch_counter += 2;
+  if (!norm) return;
   launch(finish_reduce_kernel, 1, FIN_THREADS, 0, red.p, PAIR_BLOCKS, 1, scal.p, 4);  // |r|_inf, rho_old
-  launch_counter += 4;
+  ++launch_counter;
 }
 
 // The device-side PCG loop's record, at the head of Solver::loop_buf, followed
@@ -2169,8 +2202,26 @@ static_assert(sizeof(PcgLoop) <= LOOP_REC * sizeof(double), "loop record size");
 // non-finite norm; otherwise counts the iteration and keeps the WHILE node
 // running, up to `limit`, where the host takes the history out and relaunches.
 // The loop therefore ends after at most limit - base iterations.
-__global__ void pcg_check_kernel(const double* __restrict__ scal, double* loop, cudaGraphConditionalHandle h) {
+// np partials of |r|_inf, left by residual_pair_kernel, are reduced first (0: the
+// norm is in scal[3] already); then rho_old = rho, as at the end of an iteration.
+__global__ void __launch_bounds__(RED_THREADS) pcg_check_kernel(const double* __restrict__ part, int np, double* scal,
+                                                                double* loop, cudaGraphConditionalHandle h) {
   pdl_wait();
+  __shared__ double sm[RED_THREADS / 32];
+  if (np > 0) {
+    double m = 0;
+    for (int i = threadIdx.x; i < np; i += RED_THREADS) m = fmax(m, part[i]);
+    for (int o = 16; o; o >>= 1) m = fmax(m, __shfl_down_sync(0xffffffffu, m, o));
+    if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = m;
+    __syncthreads();
+  }
+  if (threadIdx.x != 0) return;
+  if (np > 0) {
+    double m = 0;
+    for (int w = 0; w < RED_THREADS / 32; ++w) m = fmax(m, sm[w]);
+    scal[3] = m;
+    scal[1] = scal[0];
+  }
   PcgLoop* st = reinterpret_cast<PcgLoop*>(loop);
   const int it = st->it;
   const double norm = scal[3];
@@ -2257,13 +2308,13 @@ bool Solver::build_loop_graph() {
   if (!h_loop) SGS_CUDA(cudaMallocHost(&h_loop, (LOOP_REC + LOOP_HIST) * sizeof(double)));
   loop_graph = while_graph(
       [&](cudaGraphConditionalHandle h) {  // the test before the first iteration
-        launch(pcg_check_kernel, 1, 1, 0, (const double*)scal.p, loop_buf.p, h);
+        launch(pcg_check_kernel, 1, RED_THREADS, 0, red.p, 0, scal.p, loop_buf.p, h);
       },
       [&](cudaGraphConditionalHandle h) {
         const long before = launch_counter;
-        record_iteration();
+        record_iteration(false);
         launches_per_iteration = launch_counter - before;
-        launch(pcg_check_kernel, 1, 1, 0, (const double*)scal.p, loop_buf.p, h);
+        launch(pcg_check_kernel, 1, RED_THREADS, 0, red.p, PAIR_BLOCKS, scal.p, loop_buf.p, h);
         launch_counter += 2;  // the two tests
       },
       &loop_note);
@@ -2341,6 +2392,13 @@ void Solver::solve() {
   project_null<double>(l0, f.p);
   linf(f.p, nullptr);
   stage_residual();
+  if (packed0() && !P.disable_mg) {  // each V-cycle of the loop finds its packed iterate cleared
+    if (mixed())
+      launch(reset_u4_kernel<float>, blocks_for(N, 256), 256, 0, L32[0]->u4.p, Edev<float>(), N);
+    else
+      launch(reset_u4_kernel<double>, blocks_for(N, 256), 256, 0, l0.u4.p, Edev<double>(), N);
+    ++launch_counter;
+  }
   // The loop on the device: one graph launch runs iterations until the test
   // stops them (or pauses at the history buffer's end).  With an inner bottom
   // solve, whose iteration count is decided on the host, or without
@@ -2381,7 +2439,7 @@ void Solver::solve() {
       cudaGraph_t g;
       long before = launch_counter;
       SGS_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-      record_iteration();
+      record_iteration(true);
       SGS_CUDA(cudaStreamEndCapture(stream, &g));
       SGS_CUDA(cudaGraphInstantiate(&iter_graph, g, 0));
       SGS_CUDA(cudaGraphDestroy(g));
@@ -2400,7 +2458,7 @@ void Solver::solve() {
         SGS_CUDA(cudaGraphLaunch(iter_graph, stream));
         solve_launches += launches_per_iteration;
       } else {
-        record_iteration();
+        record_iteration(true);
       }
     }
   }
@@ -2411,7 +2469,7 @@ void Solver::solve() {
   }
   if (!std::isfinite(norm)) throw CudaError("non-finite residual", SGS_ERR_BREAKDOWN);
   final_residual = norm;
-  launch(add_kernel, blocks_for(n3, 256), 256, 0, x.p, ubk.p, n3);
+  launch(finish_solution_kernel, blocks_for(n3, 256), 256, 0, x.p, s.p, ubk.p, scal.p, n3, fr);
   ++launch_counter;
   SGS_CUDA(cudaEventRecord(ev_end, stream));
   SGS_CUDA(cudaGetLastError());
