@@ -259,6 +259,38 @@ static double* cell_scratch(int slot, size_t count) {
   return c.p[slot];
 }
 
+// Pinned blocks of PINNED_BYTES for the solvers' scalar mirrors, kept for the
+// process: page-locking and releasing one takes 2 ms, more than a small solve's
+// whole set-up.  A block belongs to one solver at a time; at most PINNED_KEEP
+// free ones are kept (16 KB each), the rest go back to the system.
+constexpr size_t PINNED_BYTES = 16384, PINNED_KEEP = 64;
+static std::mutex g_pinned_mutex;
+static std::vector<void*> g_pinned;
+static void* pinned_take() {
+  {
+    std::lock_guard<std::mutex> lock(g_pinned_mutex);
+    if (!g_pinned.empty()) {
+      void* p = g_pinned.back();
+      g_pinned.pop_back();
+      return p;
+    }
+  }
+  void* p = nullptr;
+  SGS_CUDA(cudaHostAlloc(&p, PINNED_BYTES, cudaHostAllocPortable));
+  return p;
+}
+static void pinned_give(void* p) {
+  if (!p) return;
+  {
+    std::lock_guard<std::mutex> lock(g_pinned_mutex);
+    if (g_pinned.size() < PINNED_KEEP) {
+      g_pinned.push_back(p);
+      return;
+    }
+  }
+  cudaFreeHost(p);
+}
+
 // Tables of a level's boundary-band groups (band_group.cuh), shared by the
 // precisions of the level.
 struct BandTables {
@@ -338,8 +370,9 @@ class Solver {
     if (ev_end) cudaEventDestroy(ev_end);
     if (iter_graph) cudaGraphExecDestroy(iter_graph);
     if (loop_graph) cudaGraphExecDestroy(loop_graph);
-    if (h_scal) cudaFreeHost(h_scal);
-    if (h_loop) cudaFreeHost(h_loop);
+    if (stream) cudaStreamSynchronize(stream);  // no copy into the pinned mirrors is left
+    pinned_give(h_scal);
+    pinned_give(h_loop);
     if (stream) cudaStreamDestroy(stream);
   }
 
@@ -414,7 +447,7 @@ class Solver {
       SGS_CUDA(cudaGetSymbolAddress(&p, g_sensitivity_partials));
       static_partials = static_cast<double*>(p);
     }
-    SGS_CUDA(cudaMallocHost(&h_scal, 16 * sizeof(double)));
+    h_scal = static_cast<double*>(pinned_take());
     using clk = std::chrono::steady_clock;
     auto t0 = clk::now();
     auto mark = [&](double* slot) {
@@ -2305,7 +2338,8 @@ bool Solver::build_loop_graph() {
   if (loop_graph) return true;
   if (loop_unavailable) return false;
   if (!loop_buf.p) loop_buf.alloc(LOOP_REC + LOOP_HIST);
-  if (!h_loop) SGS_CUDA(cudaMallocHost(&h_loop, (LOOP_REC + LOOP_HIST) * sizeof(double)));
+  static_assert((LOOP_REC + LOOP_HIST) * sizeof(double) <= PINNED_BYTES, "loop record size");
+  if (!h_loop) h_loop = static_cast<double*>(pinned_take());
   loop_graph = while_graph(
       [&](cudaGraphConditionalHandle h) {  // the test before the first iteration
         launch(pcg_check_kernel, 1, RED_THREADS, 0, red.p, 0, scal.p, loop_buf.p, h);
