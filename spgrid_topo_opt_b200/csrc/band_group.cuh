@@ -271,7 +271,7 @@ __global__ void __launch_bounds__(BG_THREADS, 1) band0_group_kernel(
         const int i = neighbour27(nbr, g, q);
         if (i >= 0) {
           if (PACKED) {
-            const V v = u4[i];
+            const V v = u4[packed_index(i)];
             w0 = s0 * v.x, w1 = s1 * v.y, w2 = s2 * v.z;
           } else {
             w0 = s0 * u[i], w1 = s1 * u[i + N], w2 = s2 * u[i + 2 * N];
@@ -289,7 +289,7 @@ __global__ void __launch_bounds__(BG_THREADS, 1) band0_group_kernel(
 #pragma unroll
       for (int q = 0; q < 3; ++q) red[q] += __shfl_xor_sync(0xffffffffu, red[q], o);
     if (on && I == 0) {
-      if (PACKED) su[s] = u4[g];
+      if (PACKED) su[s] = u4[packed_index(g)];
       else su[s] = Pack4<T>::make(u[g], u[g + N], u[g + 2 * N], T(0));
 #pragma unroll
       for (int q = 0; q < 3; ++q) sb[s * 3 + q] = b[g + q * N] - red[q] * dx;
@@ -297,7 +297,7 @@ __global__ void __launch_bounds__(BG_THREADS, 1) band0_group_kernel(
   }
   for (int h = threadIdx.x; h < hcount[rank]; h += BG_THREADS) {
     const int g = hnode[rank * S * BG_CTAS + h];
-    if (PACKED) su[S + h] = u4[g];
+    if (PACKED) su[S + h] = u4[packed_index(g)];
     else su[S + h] = Pack4<T>::make(u[g], u[g + N], u[g + 2 * N], T(0));
   }
   __syncthreads();  // a pass reads tables that other warps of the CTA filled before its barrier completes
@@ -376,7 +376,7 @@ __global__ void __launch_bounds__(BG_THREADS, 1) band0_group_kernel(
     if (g == BG_NONE) continue;
     const V v = su[s];
     if (PACKED) {
-      u4[g] = v;
+      u4[packed_index(g)] = v;
     } else {
       u[g] = v.x;
       u[g + N] = v.y;

@@ -93,7 +93,7 @@ struct Level {
   DevBuf<int> sgs_list;
   int sgs_off[17] = {0};
   // level 0 of the V-cycle (mixed and FP64 modes): the iterate packed as (u, E) per
-  // node, followed by one all-zero pad block (index nb) that nbrz names for missing neighbours
+  // node (slots in packed_index order), followed by one all-zero pad block (index nb) that nbrz names for missing neighbours
   DevBuf<typename Pack4<T>::type> u4;
   DevBuf<int> nbrz;
 };
@@ -142,7 +142,7 @@ template <typename T>
 __global__ void pack_u4_kernel(typename Pack4<T>::type* __restrict__ u4, const T* __restrict__ u, const T* __restrict__ E,
                                long N) {
   const long i = long(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i < N) u4[i] = Pack4<T>::make(u[i], u[i + N], u[i + 2 * N], E[i]);
+  if (i < N) u4[packed_index(i)] = Pack4<T>::make(u[i], u[i + N], u[i + 2 * N], E[i]);
 }
 
 // Node lists of the level-0 Gauss-Seidel passes, built on the device (see
@@ -1690,7 +1690,7 @@ __global__ void precond_out4_kernel(const typename Pack4<T>::type* __restrict__ 
   double s = 0;
   for (long i = long(blockIdx.x) * blockDim.x + threadIdx.x; i < N; i += long(gridDim.x) * blockDim.x) {
     const uint32_t fl = flags[i];
-    const auto z = z4[i];
+    const auto z = z4[packed_index(i)];
     const double zc[3] = {double(z.x), double(z.y), double(z.z)};
 #pragma unroll
     for (int v = 0; v < 3; ++v) {
@@ -1766,7 +1766,8 @@ __global__ void __launch_bounds__(RED_THREADS, 4) rho_pair_kernel(const typename
   for (long p = long(blockIdx.x) * blockDim.x + threadIdx.x; p < P; p += long(gridDim.x) * blockDim.x) {
     const uint2 fl = reinterpret_cast<const uint2*>(flags)[p];
     if (!((fl.x | fl.y) & ACTIVE_NODE)) continue;
-    const auto za = z4[2 * p], zb = z4[2 * p + 1];
+    const long at = packed_index(2 * p);
+    const auto za = z4[at], zb = z4[at + packed_z(1)];
     const double zc[2][3] = {{double(za.x), double(za.y), double(za.z)}, {double(zb.x), double(zb.y), double(zb.z)}};
 #pragma unroll
     for (int v = 0; v < 3; ++v) {
@@ -1796,12 +1797,13 @@ __global__ void __launch_bounds__(RED_THREADS, 4) direction_pair_kernel(double* 
     if (!((fl.x | fl.y) & ACTIVE_NODE)) continue;
     double zc[2][3];
     if (PACKED) {
-      auto za = z4[2 * p], zb = z4[2 * p + 1];
+      const long at = packed_index(2 * p);
+      auto za = z4[at], zb = z4[at + packed_z(1)];
       zc[0][0] = za.x, zc[0][1] = za.y, zc[0][2] = za.z;
       zc[1][0] = zb.x, zc[1][1] = zb.y, zc[1][2] = zb.z;
       za.x = za.y = za.z = zb.x = zb.y = zb.z = T(0);
-      z4[2 * p] = za;
-      z4[2 * p + 1] = zb;
+      z4[at] = za;
+      z4[at + packed_z(1)] = zb;
 #pragma unroll
       for (int v = 0; v < 3; ++v) {
         if (!(fl.x & ACTIVE_NODE) || (fl.x & (DIR_X << v))) zc[0][v] = 0;

@@ -102,7 +102,7 @@ __device__ __forceinline__ void tc_prefetch(int bi, const int* nb27, float4* hal
     const int lx = sx - 1, ly = sy - 1, lz = sz - 1;
     const int dxb = lx < 0 ? 0 : (lx > 3 ? 2 : 1), dyb = ly < 0 ? 0 : (ly > 3 ? 2 : 1), dzb = lz < 0 ? 0 : (lz > 7 ? 2 : 1);
     const int nb = nb27[dxb * 9 + dyb * 3 + dzb];
-    tc_cp16(halo + h, u4 + (long(nb) * 128 + ((lx & 3) << 5) + ((ly & 3) << 3) + (lz & 7)));
+    tc_cp16(halo + h, u4 + (long(nb) * 128 + packed_x(lx & 3) + packed_y(ly & 3) + packed_z(lz & 7)));
   }
   if (OP == OP_RES && threadIdx.x < 96) {  // 3 planes x 32 chunks of 4 floats
     const int v = threadIdx.x >> 5, c = threadIdx.x & 31;
