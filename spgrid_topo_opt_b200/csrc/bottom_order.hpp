@@ -28,6 +28,13 @@ struct BottomOrder {
   std::vector<int> list;                   // concatenated: the tiles step K touches, ascending, without K
   std::vector<int> first;                  // step K's are list[first[K]] .. list[first[K + 1]]
   std::vector<int> below;                  // how many of them are smaller than K
+  // the application: for each phase the row tiles and, per tile, the column
+  // ranges [c0, c1) of its nonzero tiles (range k of row i: at[first[i] + k])
+  struct Phase {
+    std::vector<int> tiles, first, ranges;
+  };
+  Phase phase[3];
+  bool single = true;                      // one leaf: phase 0 alone, with the full inverse
 
   void build(int tile_size) {
     tile = tile_size;
@@ -36,11 +43,16 @@ struct BottomOrder {
     ld = 0;
     std::vector<int> all(at.size());
     for (size_t i = 0; i < all.size(); ++i) all[i] = int(i);
+    leaf_of.clear();
+    leaves = 0;
     dissect(all);
+    single = leaves <= 1;
     symbolic();
   }
 
  private:
+  std::vector<int> leaf_of;                // tile -> leaf, -1 for a separator's tiles
+  int leaves = 0;
   // the axis of the largest extent of `nodes` and its range
   int longest(const std::vector<int>& nodes, int* lo, int* hi) const {
     int best = 0;
@@ -51,7 +63,7 @@ struct BottomOrder {
     }
     return best;
   }
-  void place(std::vector<int>& nodes, int axis) {
+  void place(std::vector<int>& nodes, int axis, bool leaf) {
     const int b = (axis + 1) % 3, c = (axis + 2) % 3;
     std::sort(nodes.begin(), nodes.end(), [&](int i, int j) {
       const auto &p = at[size_t(i)], &q = at[size_t(j)];
@@ -64,12 +76,14 @@ struct BottomOrder {
       ld += 3;
     }
     while (ld % tile) pad.push_back(int(ld++));
+    leaf_of.resize(size_t(ld / tile), leaf ? leaves : -1);
+    leaves += leaf;
   }
   void dissect(std::vector<int>& nodes) {
     if (nodes.empty()) return;
     int lo = 0, hi = 0;
     const int axis = longest(nodes, &lo, &hi);
-    if (3 * long(nodes.size()) <= LEAF_UNKNOWNS || hi - lo < 2) return place(nodes, axis);
+    if (3 * long(nodes.size()) <= LEAF_UNKNOWNS || hi - lo < 2) return place(nodes, axis, true);
     // the plane that splits the nodes most evenly
     std::vector<long> count(size_t(hi - lo + 1), 0);
     for (int i : nodes) ++count[size_t(at[size_t(i)][size_t(axis)] - lo)];
@@ -88,13 +102,14 @@ struct BottomOrder {
     dissect(side[0]);
     dissect(side[1]);
     int l2 = 0, h2 = 0;
-    if (!side[2].empty()) place(side[2], longest(side[2], &l2, &h2));
+    if (!side[2].empty()) place(side[2], longest(side[2], &l2, &h2), false);
   }
-  // tiles that each Gauss-Jordan step touches: row K's nonzero tiles S; the step
-  // fills all tiles of S x S
+  // tiles that each Gauss-Jordan step touches: row K's nonzero tiles S (a
+  // separator's: separators only); the step fills all tiles of S x S
   void symbolic() {
     const int nt = int(ld / tile);
     std::vector<std::vector<char>> on(size_t(nt), std::vector<char>(size_t(nt), 0));
+    for (int K = 0; K < nt; ++K) on[size_t(K)][size_t(K)] = 1;
     if (!at.empty()) {
       int lo[3], dim[3];
       for (int a = 0; a < 3; ++a) {
@@ -121,7 +136,7 @@ struct BottomOrder {
       int low = 0;
       std::vector<int> S;
       for (int J = 0; J < nt; ++J)
-        if (J != K && on[size_t(K)][size_t(J)]) {
+        if (J != K && on[size_t(K)][size_t(J)] && (leaf_of[size_t(K)] >= 0 || leaf_of[size_t(J)] < 0)) {
           S.push_back(J);
           low += J < K;
         }
@@ -130,6 +145,22 @@ struct BottomOrder {
       list.insert(list.end(), S.begin(), S.end());
       first.push_back(int(list.size()));
       below.push_back(low);
+    }
+    for (int f = 0; f < 3; ++f) {
+      Phase& p = phase[f];
+      p = Phase();
+      p.first.push_back(0);
+      for (int I = 0; I < nt; ++I) {
+        const bool leaf = leaf_of[size_t(I)] >= 0;
+        if ((f == 1 && leaf) || (f == 2 && !leaf)) continue;
+        p.tiles.push_back(I);
+        for (int J = 0; J < nt; ++J) {
+          if (!on[size_t(I)][size_t(J)] || (leaf_of[size_t(J)] >= 0) != (f == 0)) continue;
+          if (int(p.ranges.size()) > 2 * p.first.back() && p.ranges.back() == J * tile) p.ranges.back() += tile;
+          else p.ranges.insert(p.ranges.end(), {J * tile, (J + 1) * tile});
+        }
+        p.first.push_back(int(p.ranges.size() / 2));
+      }
     }
   }
 };

@@ -549,59 +549,69 @@ __global__ void bottom_gather_kernel(const int* __restrict__ node_pos, const T* 
   }
 }
 
-// y = M x, one warp per row, written to the level's field: row r is entry
-// out[r] of u (-1: padding)
-template <typename T>
-__global__ void gemv_kernel(const double* __restrict__ M, long ld, long n, const double* __restrict__ x,
-                            const int* __restrict__ out, T* __restrict__ u) {
-  const long row = (long(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  const int to = row < n ? out[row] : -1;
+// One phase of the bottom's application (BottomOrder), one warp per row over the
+// row tile's column ranges, FP64 sums (TM float: the FP32 copy of the matrix that
+// the mixed V-cycle applies).  Row r is entry out[r] of the level's field u (-1:
+// padding).  PHASE 0: y = M x over the leaves' columns (plus x on the separators);
+// SINGLE: straight to u.  PHASE 1: xs = M y on the separators.  PHASE 2: u = y +
+// M xs on the leaves.  Bound by HBM: every entry is read once per application.
+template <typename TM>
+struct MatrixVec;
+template <>
+struct MatrixVec<double> {
+  static constexpr int W = 2;
+  static __device__ __forceinline__ double dot(const double* m, const double* v, double s) {
+    const double2 a = __ldcs(reinterpret_cast<const double2*>(m)), w = *reinterpret_cast<const double2*>(v);
+    return fma(a.y, w.y, fma(a.x, w.x, s));
+  }
+};
+template <>
+struct MatrixVec<float> {
+  static constexpr int W = 4;
+  static __device__ __forceinline__ double dot(const float* m, const double* v, double s) {
+    const float4 a = __ldcs(reinterpret_cast<const float4*>(m));
+    const double2 w0 = reinterpret_cast<const double2*>(v)[0], w1 = reinterpret_cast<const double2*>(v)[1];
+    return fma(double(a.w), w1.y, fma(double(a.z), w1.x, fma(double(a.y), w0.y, fma(double(a.x), w0.x, s))));
+  }
+};
+constexpr int APPLY_ROWS = 8;  // rows per CTA of 256 threads
+template <typename TM, typename T, int PHASE, bool SINGLE>
+__global__ void __launch_bounds__(256) bottom_apply_kernel(const TM* __restrict__ M, long ld,
+                                                           const int* __restrict__ tiles, const int* __restrict__ first,
+                                                           const int* __restrict__ ranges, const double* __restrict__ x,
+                                                           double* y, double* xs, const int* __restrict__ out,
+                                                           const int* __restrict__ separator, T* __restrict__ u) {
+  constexpr int PER = SGJ / APPLY_ROWS;
+  const int k = blockIdx.x / PER, lane = threadIdx.x & 31;
+  const long row = long(tiles[k]) * SGJ + (blockIdx.x % PER) * APPLY_ROWS + (threadIdx.x >> 5);
+  const int r0 = first[k], r1 = first[k + 1], to = out[row];
   pdl_wait();
   if (to < 0) return;
-  const double2* m = reinterpret_cast<const double2*>(M + row * ld);
-  const double2* v = reinterpret_cast<const double2*>(x);
+  const TM* m = M + row * ld;
+  const double* v = PHASE == 0 ? x : (PHASE == 1 ? y : xs);
+  constexpr int W = MatrixVec<TM>::W, STEP = 32 * W;
   double s0 = 0, s1 = 0;
-#pragma unroll 4
-  for (long c = lane; c < n / 2; c += 32) {
-    const double2 a = __ldcs(m + c), w = v[c];
-    s0 = fma(a.x, w.x, s0);
-    s1 = fma(a.y, w.y, s1);
+  for (int r = r0; r < r1; ++r) {
+    int c = ranges[2 * r] + lane * W;
+    const int end = ranges[2 * r + 1];  // ranges are multiples of the tile, 128 columns
+    for (; c + STEP < end; c += 2 * STEP) {
+      s0 = MatrixVec<TM>::dot(m + c, v + c, s0);
+      s1 = MatrixVec<TM>::dot(m + c + STEP, v + c + STEP, s1);
+    }
+    if (c < end) s0 = MatrixVec<TM>::dot(m + c, v + c, s0);
   }
   double s = s0 + s1;
   for (int o = 16; o; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-  if (lane == 0) u[to] = T(s);
-}
-
-// y = M x with an FP32 copy of M (ld a multiple of 128, rows 16-byte aligned),
-// 32 rows per CTA of 1024 threads, one warp per row.  x is staged once per CTA
-// in shared memory as FP32 (exact: in mixed precision it is gathered from an
-// FP32 right-hand side), so the loop streams only M.
-constexpr int GEMV32_ROWS = 32;
-__global__ void __launch_bounds__(1024) gemv32_kernel(const float* __restrict__ M, long ld, long n,
-                                                      const double* __restrict__ x, const int* __restrict__ out,
-                                                      float* __restrict__ u) {
-  extern __shared__ float4 xs4[];
-  float* xs = reinterpret_cast<float*>(xs4);
-  pdl_wait();
-  for (long c = threadIdx.x; c < n; c += blockDim.x) xs[c] = float(x[c]);
-  __syncthreads();
-  const long row = long(blockIdx.x) * GEMV32_ROWS + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (row >= n) return;
-  const float4* m = reinterpret_cast<const float4*>(M + row * ld);
-  float s0 = 0.f, s1 = 0.f;
-  for (long c = lane; c < n / 4; c += 32) {
-    const float4 a = __ldcs(m + c);  // read once per application: do not keep it in L2
-    const float4 v = xs4[c];
-    s0 = fmaf(a.x, v.x, s0);
-    s1 = fmaf(a.y, v.y, s1);
-    s0 = fmaf(a.z, v.z, s0);
-    s1 = fmaf(a.w, v.w, s1);
+  if (lane != 0) return;
+  if (PHASE == 0) {
+    if (SINGLE) u[to] = T(s);
+    else y[row] = separator[tiles[k]] ? x[row] + s : s;
+  } else if (PHASE == 1) {
+    xs[row] = s;
+    u[to] = T(s);
+  } else {
+    u[to] = T(y[row] + s);
   }
-  double s = double(s0) + double(s1);
-  for (int o = 16; o; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-  if (lane == 0 && out[row] >= 0) u[out[row]] = float(s);
 }
 
 }  // namespace sgs

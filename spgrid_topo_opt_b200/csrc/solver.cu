@@ -106,7 +106,8 @@ struct Bottom {
   BottomOrder order;
   std::vector<int32_t> ordered_nodes;  // the nodes `order` was made for
   DevBuf<int> tiles, pad;              // BottomOrder::list and pad on the device
-  DevBuf<double> Minv, xb;
+  DevBuf<int> phase_tiles[3], phase_first[3], phase_ranges[3], separator;  // BottomOrder::phase; tile is a separator's
+  DevBuf<double> Minv, xb, y, xs;
   DevBuf<float> Minv32;  // mixed precision: the FP32 V-cycle applies an FP32 copy of Minv
 };
 
@@ -1002,6 +1003,14 @@ class Solver {
       for (size_t k = 0; k < dof_node.size(); ++k)
         for (int v = 0; v < 3; ++v) row_out[size_t(o.pos[k] + v)] = dof_node[k] + v * int(d.N);
       bottom.row_out.upload(row_out, stream);
+      std::vector<int32_t> separator(size_t(o.ld / SGJ), 0);
+      for (int t : o.phase[1].tiles) separator[size_t(t)] = 1;
+      bottom.separator.upload(separator, stream);
+      for (int f = 0; f < 3; ++f) {
+        bottom.phase_tiles[f].upload(o.phase[f].tiles, stream);
+        bottom.phase_first[f].upload(o.phase[f].first, stream);
+        bottom.phase_ranges[f].upload(o.phase[f].ranges, stream);
+      }
       bottom.node_pos.upload(node_pos, stream);
       bottom.tiles.upload(o.list, stream);
       bottom.pad.upload(o.pad, stream);
@@ -1011,6 +1020,10 @@ class Solver {
     bottom.ld = bottom.order.ld;
     bottom.xb.alloc(size_t(bottom.ld));
     bottom.xb.zero(stream);
+    for (DevBuf<double>* v : {&bottom.y, &bottom.xs}) {
+      v->alloc(bottom.order.single ? 0 : size_t(bottom.ld));
+      v->zero(stream);
+    }
     if (bottom.n == 0) return;
     bottom.Minv.alloc(size_t(bottom.ld) * bottom.ld);
     bottom.Minv.zero(stream);
@@ -1023,9 +1036,6 @@ class Solver {
     SGS_CUDA(cudaGetLastError());
     invert_bottom(bottom.Minv.p, bottom.ld);
     if (mixed()) {
-      // the most that any session's bottom needs (the attribute is the kernel's, not the session's)
-      SGS_CUDA(cudaFuncSetAttribute(gemv32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    int(std::max(bottom.ld, 28672L) * sizeof(float))));
       bottom.Minv32.alloc(bottom.Minv.n);
       convert_kernel<float, double><<<blocks_for(long(bottom.Minv.n), 256), 256, 0, stream>>>(
           bottom.Minv32.p, bottom.Minv.p, long(bottom.Minv.n));
@@ -1323,6 +1333,21 @@ class Solver {
     bottom_dense<T>(l, round_ref());
   }
 
+  template <typename TM, typename T>
+  void bottom_apply(const TM* M, T* u) {
+    auto phase = [&](auto kernel, int f) {
+      if (bottom.phase_tiles[f].n == 0) return;
+      launch(kernel, unsigned(bottom.phase_tiles[f].n * (SGJ / APPLY_ROWS)), 256, 0, M, bottom.ld, bottom.phase_tiles[f].p,
+             bottom.phase_first[f].p, bottom.phase_ranges[f].p, bottom.xb.p, bottom.y.p, bottom.xs.p, bottom.row_out.p,
+             bottom.separator.p, u);
+      ++launch_counter;
+    };
+    if (bottom.order.single) return phase(bottom_apply_kernel<TM, T, 0, true>, 0);
+    phase(bottom_apply_kernel<TM, T, 0, false>, 0);
+    phase(bottom_apply_kernel<TM, T, 1, false>, 1);
+    phase(bottom_apply_kernel<TM, T, 2, false>, 2);
+  }
+
   // u = M^-1 b on the deepest level (nodes without unknowns keep b)
   template <typename T>
   void bottom_dense(int l, bool round) {
@@ -1331,14 +1356,10 @@ class Solver {
     launch(bottom_gather_kernel<T>, blocks_for(d.N, 256), 256, 0, bottom.node_pos.p, d.b.p, d.N, bottom.xb.p, d.u.p);
     ++launch_counter;
     if (bottom.ndof_nodes > 0) {
-      if constexpr (sizeof(T) == 4) {  // the FP32 V-cycle applies the FP32 copy
-        launch(gemv32_kernel, blocks_for(bottom.ld, GEMV32_ROWS), 1024, size_t(bottom.ld) * sizeof(float),
-               bottom.Minv32.p, bottom.ld, bottom.ld, bottom.xb.p, bottom.row_out.p, d.u.p);
-      } else {
-        launch(gemv_kernel<T>, blocks_for(bottom.ld * 32, 256), 256, 0, bottom.Minv.p, bottom.ld, bottom.ld, bottom.xb.p,
-               bottom.row_out.p, d.u.p);
-      }
-      ++launch_counter;
+      if constexpr (sizeof(T) == 4)  // the FP32 V-cycle applies the FP32 copy
+        bottom_apply(bottom.Minv32.p, d.u.p);
+      else
+        bottom_apply(bottom.Minv.p, d.u.p);
     }
     if (round) round3(d, d.u.p);
   }
