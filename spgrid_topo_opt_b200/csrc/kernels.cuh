@@ -72,6 +72,14 @@ struct KcReg {
   }
 };
 
+// The level-0 operator at large sizes streams from HBM, whose latency its
+// resident warps do not cover: a CTA asks for the data of the one that will
+// follow it on the chip (about one wave of CTAs ahead) to be brought into L2
+// (1024^3 FP32 residual 1402 -> 1112 us).  The Gauss-Seidel passes, whose gathers
+// keep more lines in flight, lost by it (1476 -> 1686 us a sweep).
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+constexpr int WAVE_SMS = 148;
+
 // the packed node record of level 0: (u_x, u_y, u_z, E)
 template <typename T>
 struct Pack4;
@@ -134,15 +142,15 @@ __device__ __forceinline__ void pdl_wait() {
 // 64 idle.  Cells without material (E = 0) skip the modal part.
 // PACKED: the iterate is the record u4 = (u, E) with the neighbour table nbrz
 // (a zero pad block for missing blocks), else the planes of u, E and nbr (-1).
-// Bound by shared-memory bandwidth (66 KB a block in FP64) and, in FP64, the FMA
-// pipe.  At 1024^3 (340713 blocks): FP64 matvec 2240 -> 2169 us, FP32 residual
-// 1348 -> 1188 us (nodal form -> this).
+// Bound by latency: a CTA's five steps are a chain of loads, about 15 dependent
+// operations and a barrier each, and registers allow 5 CTAs an SM in FP64, 9 in
+// FP32 (4 / 8: 12% slower in FP64; 6 / 10, with spills: 23%).  At 1024^3 (340713
+// blocks), nodal form -> this: FP64 matvec 2240 -> 2010 us, FP32 residual 1348 ->
+// 962 us; 48^3 14.3 -> 8.0 us and 11.9 -> 9.0 us.
 // ---------------------------------------------------------------------------
 enum { OP_KU = 0, OP_RES = 1, OP_KUP = 2 };
 
-// halo geometry: nodes [-1,4]x[-1,4]x[-1,8] (6x6x10), cells [-1,3]x[-1,3]x[-1,7] (5x5x9)
-constexpr int HU = 360, HE = 225;
-constexpr int MODAL_THREADS = 96, MODAL_BLOCKS = 2, MODAL_COLS = 45;
+constexpr int MODAL_THREADS = 96, MODAL_BLOCKS = 2;
 
 // dx/16 times the Lame parameters and their modal combinations
 template <typename T>
@@ -154,64 +162,73 @@ struct ModalCoef {
   }
 };
 
-// one value to shared memory with cp.async (zero where !on): a thread's whole
-// share of a halo is in flight at once
-template <typename T>
-__device__ __forceinline__ void stage_async(T* smem, const T* gmem, bool on) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n" ::"r"(unsigned(__cvta_generic_to_shared(smem))), "l"(gmem),
-               "n"(int(sizeof(T))), "r"(on ? int(sizeof(T)) : 0)
-               : "memory");
-}
-
 template <typename T, int OP, bool PACKED>
-__global__ void __launch_bounds__(MODAL_THREADS, sizeof(T) == 8 ? 5 : 8) level0_modal_kernel(
+__global__ void __launch_bounds__(MODAL_THREADS, sizeof(T) == 8 ? 5 : 9) level0_modal_kernel(
     int nblocks, const int* __restrict__ nbr, const T* __restrict__ E, const T* __restrict__ u,
     const typename Pack4<T>::type* __restrict__ u4, const T* __restrict__ b, T* __restrict__ out, long N,
     ModalCoef<T> K, const uint32_t* __restrict__ flags, double* __restrict__ part) {
-  constexpr int BUFS = sizeof(T) == 8 ? 1 : 2;  // exchange buffers: one more barrier a plane, but more CTAs, in FP64
-  __shared__ T su[MODAL_BLOCKS][3][HU];
-  __shared__ T sE[MODAL_BLOCKS][HE];
-  __shared__ T sx[BUFS][12][MODAL_THREADS];
-  __shared__ int snb[MODAL_BLOCKS * 27];
+  __shared__ T sx[2][12][MODAL_THREADS];
   const int t = threadIdx.x;
   const int b0 = blockIdx.x * MODAL_BLOCKS;
-  if (t < MODAL_BLOCKS * 27) snb[t] = b0 + t / 27 < nblocks ? nbr[long(b0) * 27 + t] : -1;
-  pdl_wait();
-  __syncthreads();
-  for (int h2 = t; h2 < MODAL_BLOCKS * HU; h2 += MODAL_THREADS) {
-    const int k = h2 / HU, h = h2 % HU;
-    const int sx_ = h / 60, sy = (h / 10) % 6, sz = h % 10;
-    const int lx = sx_ - 1, ly = sy - 1, lz = sz - 1;
-    const int dxb = lx < 0 ? 0 : (lx > 3 ? 2 : 1), dyb = ly < 0 ? 0 : (ly > 3 ? 2 : 1), dzb = lz < 0 ? 0 : (lz > 7 ? 2 : 1);
-    const int nb = snb[k * 27 + dxb * 9 + dyb * 3 + dzb];
-    const long i = nb < 0 ? 0 : long(nb) * 128 + ((lx & 3) << 5) + ((ly & 3) << 3) + (lz & 7);
-    const bool cell = sx_ < 5 && sy < 5 && sz < 9;
-    T* ce = &sE[k][cell ? (sx_ * 5 + sy) * 9 + sz : 0];
-    if (PACKED) {
-      const T* r = reinterpret_cast<const T*>(u4 + packed_index(i));
-      stage_async(&su[k][0][h], r, nb >= 0);
-      stage_async(&su[k][1][h], r + 1, nb >= 0);
-      stage_async(&su[k][2][h], r + 2, nb >= 0);
-      if (cell) stage_async(ce, r + 3, nb >= 0);
-    } else {
-      stage_async(&su[k][0][h], u + i, nb >= 0);
-      stage_async(&su[k][1][h], u + i + N, nb >= 0);
-      stage_async(&su[k][2][h], u + i + 2 * N, nb >= 0);
-      if (cell) stage_async(ce, E + i, nb >= 0);
+  // this thread's column of cells, min corners at (cy, cz) - 1 of block b0 + blk:
+  // 40 columns with cz > 0 a block, then the 5 with cz = 0 of each
+  const int rest = t - 80;
+  const int blk = t < 80 ? t / 40 : rest / 5, cy = t < 80 ? t % 40 / 8 : rest % 5, cz = t < 80 ? t % 8 + 1 : 0;
+  const bool on = t < 90 && b0 + blk < nblocks;
+  // first records of the column's four corners in the blocks behind, at and ahead of it in x
+  int at[3][4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int y = cy - 1 + (k >> 1), z = cz - 1 + (k & 1);
+    const int nb = (y < 0 ? 0 : (y > 3 ? 2 : 1)) * 3 + (z < 0 ? 0 : (z > 7 ? 2 : 1));
+    const int yz = PACKED ? packed_y(y & 3) + packed_z(z & 7) : ((y & 3) << 3) + (z & 7);
+#pragma unroll
+    for (int g = 0; g < 3; ++g) {
+      const int j = on ? __ldg(nbr + long(b0 + blk) * 27 + g * 9 + nb) : -1;
+      at[g][k] = j < 0 ? -1 : (j << 7) + yz;
     }
   }
-  asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
-  __syncthreads();
-  const int blk = t >= MODAL_COLS ? 1 : 0, col = min(t - blk * MODAL_COLS, MODAL_COLS - 1);  // lanes 90..95 idle along
-  const T* un = &su[blk][0][(col / 9) * 10 + col % 9];
-  const T* ec = &sE[blk][col];
-  // modes 1, z, y, yz of a node plane's face
-  auto face = [&](int plane, T (&m)[4][3]) {
+  {
+    constexpr int PER = 128 / int(sizeof(T));                  // values per line
+    constexpr int UL = (PACKED ? 4 : 3) * 128 / PER, EL = PACKED ? 0 : 128 / PER, BL = OP == OP_RES ? 3 * 128 / PER : 0;
+    const int ahead = b0 + MODAL_BLOCKS * WAVE_SMS * (sizeof(T) == 8 ? 5 : 9);
+    for (int l = t; l < MODAL_BLOCKS * (UL + EL + BL); l += MODAL_THREADS) {
+      const int k = l / (UL + EL + BL), j = l % (UL + EL + BL);
+      if (ahead + k >= nblocks) continue;
+      const long first = long(ahead + k) * 128;
+      if (j < UL) prefetch_l2(PACKED ? reinterpret_cast<const T*>(u4 + first) + j * PER
+                                     : u + first + (j / (128 / PER)) * N + (j % (128 / PER)) * PER);
+      else if (j < UL + EL) prefetch_l2(E + first + (j - UL) * PER);
+      else prefetch_l2(b + first + ((j - UL - EL) / (128 / PER)) * N + ((j - UL - EL) % (128 / PER)) * PER);
+    }
+  }
+  pdl_wait();
+  // a node plane's four corners (plane 0 and 5: one node beyond the block), and
+  // the stiffness of the cell ahead of it
+  T R[4][3], eR = 0;
+  auto fetch = [&](int plane, const int (&a)[4]) {
+    const int ox = PACKED ? packed_x((plane + 3) & 3) : ((plane + 3) & 3) << 5;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      R[k][0] = R[k][1] = R[k][2] = T(0);
+      if (k == 0) eR = T(0);
+      if (a[k] < 0) continue;
+      const int i = a[k] + ox;
+      if (PACKED) {
+        const auto r = u4[i];
+        R[k][0] = r.x, R[k][1] = r.y, R[k][2] = r.z;
+        if (k == 0) eR = r.w;
+      } else {
+        R[k][0] = u[i], R[k][1] = u[i + N], R[k][2] = u[i + 2 * N];
+        if (k == 0) eR = E[i];
+      }
+    }
+  };
+  // its modes 1, z, y, yz
+  auto face = [&](T (&m)[4][3]) {
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      const T* p = un + c * HU + plane * 60;
-      const T v00 = p[0], v01 = p[1], v10 = p[10], v11 = p[11];
-      const T s0 = v00 + v01, s1 = v10 + v11, d0 = v01 - v00, d1 = v11 - v10;
+      const T s0 = R[0][c] + R[1][c], s1 = R[2][c] + R[3][c], d0 = R[1][c] - R[0][c], d1 = R[3][c] - R[2][c];
       m[0][c] = s0 + s1;
       m[1][c] = d0 + d1;
       m[2][c] = s1 - s0;
@@ -219,15 +236,21 @@ __global__ void __launch_bounds__(MODAL_THREADS, sizeof(T) == 8 ? 5 : 8) level0_
     }
   };
   T P[4][3], H[4][3];  // the last plane's modes; the modal forces on it from the cell behind
-  face(0, P);
+  fetch(0, at[0]);
+  face(P);
+  T e = eR;
+  fetch(1, at[1]);
 #pragma unroll
   for (int k = 0; k < 4; ++k) H[k][0] = H[k][1] = H[k][2] = T(0);
   double dot = 0;
-#pragma unroll 1
-  for (int x = 0; x < 5; ++x) {  // cell x - 1, between node planes x - 1 and x (own planes are 1..4 of the halo)
+#pragma unroll
+  for (int x = 0; x < 5; ++x) {  // cell x - 1, between node planes x - 1 and x of the block (x and x + 1 here)
     T Q[4][3];
-    face(x + 1, Q);
-    const T e = ec[x * MODAL_COLS];
+    face(Q);
+    const T e_next = eR;
+    // the next plane's loads are in flight while this cell is computed
+    if (x < 3) fetch(x + 2, at[1]);
+    else if (x == 3) fetch(5, at[2]);
     if (e != T(0)) {
       T D[4][3], S1[3], S2[3], S3[3];
 #pragma unroll
@@ -274,8 +297,7 @@ __global__ void __launch_bounds__(MODAL_THREADS, sizeof(T) == 8 ? 5 : 8) level0_
       for (int k = 0; k < 4; ++k) P[k][0] = P[k][1] = P[k][2] = T(0);
     }
     if (x > 0) {  // plane x - 1 of the block is complete: corner forces to the nodes
-      T(*ex)[MODAL_THREADS] = sx[x & (BUFS - 1)];
-      if (BUFS == 1) __syncthreads();
+      T(*ex)[MODAL_THREADS] = sx[x & 1];
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
         const T e0 = H[0][c] - H[1][c], e1 = H[0][c] + H[1][c], o0 = H[2][c] - H[3][c], o1 = H[2][c] + H[3][c];
@@ -289,14 +311,15 @@ __global__ void __launch_bounds__(MODAL_THREADS, sizeof(T) == 8 ? 5 : 8) level0_
 #pragma unroll
       for (int k = 0; k < MODAL_BLOCKS; ++k) {
         if (b0 + k >= nblocks) continue;
-        const int q = k * MODAL_COLS + (y + 1) * 9 + z + 1;  // the column whose min corner is the node
-        T f = (ex[c][q] + ex[3 + c][q - 1]) + (ex[6 + c][q - 9] + ex[9 + c][q - 10]);
+        const int q = k * 40 + (y + 1) * 8 + z;  // the column whose min corner is the node, and its neighbour in z
+        const int qz = z > 0 ? q - 1 : 80 + k * 5 + y + 1;
+        T f = (ex[c][q] + ex[3 + c][qz]) + (ex[6 + c][q - 8] + ex[9 + c][z > 0 ? q - 9 : qz - 1]);
         const long node = long(b0 + k) * 128 + (x - 1) * 32 + (t & 31), g = node + c * N;
         if (OP == OP_RES) {
           f = b[g] - f;
         } else if (OP == OP_KUP) {
           if (flags[node] & (DIR_X << c)) f = 0;
-          dot += double(su[k][c][x * 60 + (y + 1) * 10 + z + 1]) * double(f);
+          dot += double(u[g]) * double(f);
         }
         out[g] = f;
       }
@@ -308,6 +331,7 @@ __global__ void __launch_bounds__(MODAL_THREADS, sizeof(T) == 8 ? 5 : 8) level0_
         H[k][c] = P[k][c];
         P[k][c] = Q[k][c];
       }
+    e = e_next;
   }
   if (OP == OP_KUP) {
 #pragma unroll
