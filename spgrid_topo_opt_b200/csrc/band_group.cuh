@@ -68,26 +68,6 @@ __device__ __forceinline__ void cluster_store(uint32_t a, double4 v) {
   asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a + 16), "d"(v.z) : "memory");
 }
 
-// Inverse of the node's 3x3 diagonal block {d0, d1, d2, d01, d02, d12} with the
-// rows of Dirichlet components replaced by the identity and then dropped (the
-// update of gs0_list4_kernel and stencil_op_kernel).
-template <typename T>
-__device__ __forceinline__ void band_inverse(T d0, T d1, T d2, T d3, T d4, T d5, uint32_t fl, T* a) {
-  const bool fx = fl & DIR_X, fy = fl & DIR_Y, fz = fl & DIR_Z;
-  if (fx) { d0 = 1; d3 = 0; d4 = 0; }
-  if (fy) { d1 = 1; d3 = 0; d5 = 0; }
-  if (fz) { d2 = 1; d4 = 0; d5 = 0; }
-  const T m11 = d1 * d2 - d5 * d5, m12 = d5 * d4 - d2 * d3, m13 = d3 * d5 - d4 * d1;
-  const T m22 = d2 * d0 - d4 * d4, m23 = d4 * d3 - d0 * d5, m33 = d0 * d1 - d3 * d3;
-  const T inv = T(1) / (d0 * m11 + d3 * m12 + d4 * m13);
-  a[0] = fx ? T(0) : m11 * inv;
-  a[1] = fy ? T(0) : m22 * inv;
-  a[2] = fz ? T(0) : m33 * inv;
-  a[3] = fx || fy ? T(0) : m12 * inv;
-  a[4] = fx || fz ? T(0) : m13 * inv;
-  a[5] = fy || fz ? T(0) : m23 * inv;
-}
-
 // global index of g's neighbour at offset (q / 9, q / 3 % 3, q % 3) - 1, or -1
 __device__ __forceinline__ int neighbour27(const int* __restrict__ nbr, int g, int q) {
   const int x = ((g >> 5) & 3) + q / 9 - 1, y = ((g >> 3) & 3) + q / 3 % 3 - 1, z = (g & 7) + q % 3 - 1;
@@ -250,7 +230,7 @@ __global__ void __launch_bounds__(BG_THREADS, 1) band0_group_kernel(
       const uint32_t fl = flags[g];
       sf[s] = fl;
       T a[6];
-      band_inverse<T>(red[0] * dx, red[1] * dx, red[2] * dx, red[3] * dx, red[4] * dx, red[5] * dx, fl, a);
+      diagonal_inverse<T>(red[0] * dx, red[1] * dx, red[2] * dx, red[3] * dx, red[4] * dx, red[5] * dx, fl, a);
 #pragma unroll
       for (int q = 0; q < 6; ++q) sd[s * 6 + q] = a[q];
     }
@@ -436,7 +416,7 @@ __global__ void __launch_bounds__(BG_THREADS, 1) bandc_group_kernel(
       const uint32_t fl = flags[g];
       const T* m = row + 13 * 9;
       T a[6];
-      band_inverse<T>(m[0], m[4], m[8], m[1], m[2], m[5], fl, a);
+      diagonal_inverse<T>(m[0], m[4], m[8], m[1], m[2], m[5], fl, a);
       sf[s] = fl;
 #pragma unroll
       for (int q = 0; q < 6; ++q) sd[s * 6 + q] = a[q];

@@ -111,6 +111,32 @@ __host__ __device__ __forceinline__ constexpr I packed_index(I g) {
   return (g & ~I(127)) | I(packed_x(e >> 5) | packed_y(e >> 3 & 3) | packed_z(e & 7));
 }
 
+// Inverse of a node's symmetric 3x3 diagonal block {00, 11, 22, 01, 02, 12}, the
+// rows of Dirichlet components replaced by the identity and then dropped.  In
+// FP32 the block is scaled by a power of two first (exact): its determinant,
+// the cube of a stiffness, underflows on coarse levels and for soft material.
+template <typename T>
+__device__ __forceinline__ void diagonal_inverse(T d0, T d1, T d2, T d3, T d4, T d5, uint32_t fl, T* a) {
+  const bool fx = fl & DIR_X, fy = fl & DIR_Y, fz = fl & DIR_Z;
+  T s = 1;
+  if (sizeof(T) == 4) {
+    s = T(__int_as_float(0x7f000000 - (__float_as_int(float(d0 + d1 + d2)) & 0x7f800000)));
+    d0 *= s, d1 *= s, d2 *= s, d3 *= s, d4 *= s, d5 *= s;
+  }
+  if (fx) { d0 = 1; d3 = 0; d4 = 0; }
+  if (fy) { d1 = 1; d3 = 0; d5 = 0; }
+  if (fz) { d2 = 1; d4 = 0; d5 = 0; }
+  const T m11 = d1 * d2 - d5 * d5, m12 = d5 * d4 - d2 * d3, m13 = d3 * d5 - d4 * d1;
+  const T m22 = d2 * d0 - d4 * d4, m23 = d4 * d3 - d0 * d5, m33 = d0 * d1 - d3 * d3;
+  const T inv = T(1) / (d0 * m11 + d3 * m12 + d4 * m13) * s;
+  a[0] = fx ? T(0) : m11 * inv;
+  a[1] = fy ? T(0) : m22 * inv;
+  a[2] = fz ? T(0) : m33 * inv;
+  a[3] = fx || fy ? T(0) : m12 * inv;
+  a[4] = fx || fz ? T(0) : m13 * inv;
+  a[5] = fy || fz ? T(0) : m23 * inv;
+}
+
 // Programmatic dependent launch: kernels of the solve are launched so that they
 // may start while their predecessor drains.  Each waits here until the
 // predecessor has completed and its writes are visible, then lets its own
@@ -463,17 +489,9 @@ __global__ void __launch_bounds__(128, MINB) gs0_list_kernel(const int* __restri
   }
   // u += D^{-1} (b - K u), Dirichlet rows replaced by the identity
   const T r0 = b[g] - f[0] * dx, r1 = b[g + N] - f[1] * dx, r2 = b[g + 2 * N] - f[2] * dx;
-  T d0 = dg[0] * dx, d1 = dg[1] * dx, d2 = dg[2] * dx, d3 = dg[3] * dx, d4 = dg[4] * dx, d5 = dg[5] * dx;
-  if (fx) { d0 = 1; d3 = 0; d4 = 0; }
-  if (fy) { d1 = 1; d3 = 0; d5 = 0; }
-  if (fz) { d2 = 1; d4 = 0; d5 = 0; }
-  const T m11 = d1 * d2 - d5 * d5, m12 = d5 * d4 - d2 * d3, m13 = d3 * d5 - d4 * d1;
-  const T m22 = d2 * d0 - d4 * d4, m23 = d4 * d3 - d0 * d5, m33 = d0 * d1 - d3 * d3;
-  const T inv = T(1) / (d0 * m11 + d3 * m12 + d4 * m13);
-  T a0 = m11 * inv, a1 = m22 * inv, a2 = m33 * inv, a3 = m12 * inv, a4 = m13 * inv, a5 = m23 * inv;
-  if (fx) { a0 = 0; a3 = 0; a4 = 0; }
-  if (fy) { a1 = 0; a3 = 0; a5 = 0; }
-  if (fz) { a2 = 0; a4 = 0; a5 = 0; }
+  T a[6];
+  diagonal_inverse<T>(dg[0] * dx, dg[1] * dx, dg[2] * dx, dg[3] * dx, dg[4] * dx, dg[5] * dx, fl, a);
+  const T a0 = a[0], a1 = a[1], a2 = a[2], a3 = a[3], a4 = a[4], a5 = a[5];
   T v0 = uc[0] + r0 * a0 + r1 * a3 + r2 * a4;
   T v1 = uc[1] + r0 * a3 + r1 * a1 + r2 * a5;
   T v2 = uc[2] + r0 * a4 + r1 * a5 + r2 * a2;
@@ -605,17 +623,9 @@ __global__ void __launch_bounds__(128, MINB) gs0_list4_kernel(const int* __restr
     }
   }
   const T r0 = b[g] - f[0] * dx, r1 = b[g + N] - f[1] * dx, r2 = b[g + 2 * N] - f[2] * dx;
-  T d0 = dg[0] * dx, d1 = dg[1] * dx, d2 = dg[2] * dx, d3 = dg[3] * dx, d4 = dg[4] * dx, d5 = dg[5] * dx;
-  if (fx) { d0 = 1; d3 = 0; d4 = 0; }
-  if (fy) { d1 = 1; d3 = 0; d5 = 0; }
-  if (fz) { d2 = 1; d4 = 0; d5 = 0; }
-  const T m11 = d1 * d2 - d5 * d5, m12 = d5 * d4 - d2 * d3, m13 = d3 * d5 - d4 * d1;
-  const T m22 = d2 * d0 - d4 * d4, m23 = d4 * d3 - d0 * d5, m33 = d0 * d1 - d3 * d3;
-  const T inv = T(1) / (d0 * m11 + d3 * m12 + d4 * m13);
-  T a0 = m11 * inv, a1 = m22 * inv, a2 = m33 * inv, a3 = m12 * inv, a4 = m13 * inv, a5 = m23 * inv;
-  if (fx) { a0 = 0; a3 = 0; a4 = 0; }
-  if (fy) { a1 = 0; a3 = 0; a5 = 0; }
-  if (fz) { a2 = 0; a4 = 0; a5 = 0; }
+  T a[6];
+  diagonal_inverse<T>(dg[0] * dx, dg[1] * dx, dg[2] * dx, dg[3] * dx, dg[4] * dx, dg[5] * dx, fl, a);
+  const T a0 = a[0], a1 = a[1], a2 = a[2], a3 = a[3], a4 = a[4], a5 = a[5];
   T v0 = uc[0] + r0 * a0 + r1 * a3 + r2 * a4;
   T v1 = uc[1] + r0 * a3 + r1 * a1 + r2 * a5;
   T v2 = uc[2] + r0 * a4 + r1 * a5 + r2 * a2;
@@ -743,17 +753,9 @@ __global__ void __launch_bounds__(128) gs0_cell_kernel(const int* __restrict__ l
     for (int q = 0; q < 9; ++q) red[q] += __shfl_xor_sync(group, red[q], o);
   if (I != 0) return;
   const T r0 = b[g] - red[0] * dx, r1 = b[g + N] - red[1] * dx, r2 = b[g + 2 * N] - red[2] * dx;
-  T d0 = red[3] * dx, d1 = red[4] * dx, d2 = red[5] * dx, d3 = red[6] * dx, d4 = red[7] * dx, d5 = red[8] * dx;
-  if (fx) { d0 = 1; d3 = 0; d4 = 0; }
-  if (fy) { d1 = 1; d3 = 0; d5 = 0; }
-  if (fz) { d2 = 1; d4 = 0; d5 = 0; }
-  const T m11 = d1 * d2 - d5 * d5, m12 = d5 * d4 - d2 * d3, m13 = d3 * d5 - d4 * d1;
-  const T m22 = d2 * d0 - d4 * d4, m23 = d4 * d3 - d0 * d5, m33 = d0 * d1 - d3 * d3;
-  const T inv = T(1) / (d0 * m11 + d3 * m12 + d4 * m13);
-  T a0 = m11 * inv, a1 = m22 * inv, a2 = m33 * inv, a3 = m12 * inv, a4 = m13 * inv, a5 = m23 * inv;
-  if (fx) { a0 = 0; a3 = 0; a4 = 0; }
-  if (fy) { a1 = 0; a3 = 0; a5 = 0; }
-  if (fz) { a2 = 0; a4 = 0; a5 = 0; }
+  T a[6];
+  diagonal_inverse<T>(red[3] * dx, red[4] * dx, red[5] * dx, red[6] * dx, red[7] * dx, red[8] * dx, fl, a);
+  const T a0 = a[0], a1 = a[1], a2 = a[2], a3 = a[3], a4 = a[4], a5 = a[5];
   T v0 = uc[0] + r0 * a0 + r1 * a3 + r2 * a4;
   T v1 = uc[1] + r0 * a3 + r1 * a1 + r2 * a5;
   T v2 = uc[2] + r0 * a4 + r1 * a5 + r2 * a2;
@@ -802,7 +804,7 @@ enum { SOP_MUL = 0, SOP_RES = 1, SOP_GS = 2 };
 // projected, which is the same because the V-cycle keeps u zero on Dirichlet
 // components (cleared levels, projected transfers and updates).
 template <typename T, int OP>
-__global__ void __launch_bounds__(256) stencil_op_kernel(const int* __restrict__ list, int count,
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 8 : 5) stencil_op_kernel(const int* __restrict__ list, int count,
                                                          const int* __restrict__ nbr,
                                                          const T* __restrict__ A, const uint32_t* __restrict__ flags,
                                                          const T* u, T* out_u, const T* __restrict__ b,
@@ -836,10 +838,10 @@ __global__ void __launch_bounds__(256) stencil_op_kernel(const int* __restrict__
     for (int k = 0; k < 9; ++k) a[k] = T(0);
   }
   const long n = nbk < 0 ? -1 : long(nbk) * 128 + ((X & 3) << 5) + ((Y & 3) << 3) + (Z & 7);
-  T d0 = 0, d1 = 0, d2 = 0, d3 = 0, d4 = 0, d5 = 0;
+  T inv[6] = {0, 0, 0, 0, 0, 0};  // off the pass's chain: before the wait
   if (OP == SOP_GS && lane == 0) {
     const T* c = A + gidx * 243 + 13 * 9;
-    d0 = c[0]; d1 = c[4]; d2 = c[8]; d3 = c[1]; d4 = c[2]; d5 = c[5];
+    diagonal_inverse<T>(c[0], c[4], c[8], c[1], c[2], c[5], fl, inv);
   }
   pdl_wait();
   // lane 0 reads its right-hand side (and in GS its own u) after the warp's
@@ -884,19 +886,9 @@ __global__ void __launch_bounds__(256) stencil_op_kernel(const int* __restrict__
     return;
   }
   const bool fx = fl & DIR_X, fy = fl & DIR_Y, fz = fl & DIR_Z;
-  if (fx) { d0 = 1; d3 = 0; d4 = 0; }
-  if (fy) { d1 = 1; d3 = 0; d5 = 0; }
-  if (fz) { d2 = 1; d4 = 0; d5 = 0; }
-  const T m11 = d1 * d2 - d5 * d5, m12 = d5 * d4 - d2 * d3, m13 = d3 * d5 - d4 * d1;
-  const T m22 = d2 * d0 - d4 * d4, m23 = d4 * d3 - d0 * d5, m33 = d0 * d1 - d3 * d3;
-  const T inv = T(1) / (d0 * m11 + d3 * m12 + d4 * m13);
-  T a0 = m11 * inv, a1 = m22 * inv, a2 = m33 * inv, a3 = m12 * inv, a4 = m13 * inv, a5 = m23 * inv;
-  if (fx) { a0 = 0; a3 = 0; a4 = 0; }
-  if (fy) { a1 = 0; a3 = 0; a5 = 0; }
-  if (fz) { a2 = 0; a4 = 0; a5 = 0; }
-  T u0 = u[gidx] + (a0 * r0 + a3 * r1 + a4 * r2);
-  T u1 = u[gidx + N] + (a3 * r0 + a1 * r1 + a5 * r2);
-  T u2 = u[gidx + 2 * N] + (a4 * r0 + a5 * r1 + a2 * r2);
+  T u0 = u[gidx] + (inv[0] * r0 + inv[3] * r1 + inv[4] * r2);
+  T u1 = u[gidx + N] + (inv[3] * r0 + inv[1] * r1 + inv[5] * r2);
+  T u2 = u[gidx + 2 * N] + (inv[4] * r0 + inv[5] * r1 + inv[2] * r2);
   if (fx) u0 = 0;
   if (fy) u1 = 0;
   if (fz) u2 = 0;
