@@ -76,7 +76,8 @@ struct KcReg {
 // resident warps do not cover: a CTA asks for the data of the one that will
 // follow it on the chip (about one wave of CTAs ahead) to be brought into L2
 // (1024^3 FP32 residual 1402 -> 1112 us).  The Gauss-Seidel passes, whose gathers
-// keep more lines in flight, lost by it (1476 -> 1686 us a sweep).
+// keep more lines in flight, lost by it (1476 -> 1686 us a sweep), as by prefetches of their
+// later gathers into L1 (1453 -> 1574 us).
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 constexpr int WAVE_SMS = 148;
 
@@ -171,8 +172,9 @@ __device__ __forceinline__ void pdl_wait() {
 // Bound by latency: a CTA's five steps are a chain of loads, about 15 dependent
 // operations and a barrier each, and registers allow 5 CTAs an SM in FP64, 9 in
 // FP32 (4 / 8: 12% slower in FP64; 6 / 10, with spills: 23%).  At 1024^3 (340713
-// blocks), nodal form -> this: FP64 matvec 2240 -> 2010 us, FP32 residual 1348 ->
-// 962 us; 48^3 14.3 -> 8.0 us and 11.9 -> 9.0 us.
+// blocks), nodal form -> this: FP64 matvec 2240 -> 1830 us, FP32 residual 1348 ->
+// 890 us; 48^3 14.3 -> 8.3 us and 11.9 -> 8.6 us.  (The operands of the node phase
+// are requested at the step's start: 2010 and 962 us when loaded where used.)
 // ---------------------------------------------------------------------------
 enum { OP_KU = 0, OP_RES = 1, OP_KUP = 2 };
 
@@ -271,6 +273,19 @@ __global__ void __launch_bounds__(MODAL_THREADS, sizeof(T) == 8 ? 5 : 9) level0_
   double dot = 0;
 #pragma unroll
   for (int x = 0; x < 5; ++x) {  // cell x - 1, between node planes x - 1 and x of the block (x and x + 1 here)
+    // what the nodes of the finished plane need besides the forces, requested early
+    const int nc = t >> 5;  // warp c sums component c of the plane's 32 nodes
+    T extra[MODAL_BLOCKS];
+    uint32_t fl[MODAL_BLOCKS];
+#pragma unroll
+    for (int k = 0; k < MODAL_BLOCKS; ++k) {
+      extra[k] = T(0);
+      fl[k] = 0;
+      if (x == 0 || OP == OP_KU || b0 + k >= nblocks) continue;
+      const long node = long(b0 + k) * 128 + (x - 1) * 32 + (t & 31);
+      extra[k] = OP == OP_RES ? b[node + nc * N] : u[node + nc * N];
+      if (OP == OP_KUP) fl[k] = flags[node];
+    }
     T Q[4][3];
     face(Q);
     const T e_next = eR;
@@ -333,7 +348,7 @@ __global__ void __launch_bounds__(MODAL_THREADS, sizeof(T) == 8 ? 5 : 9) level0_
         ex[9 + c][t] = e1 + o1;
       }
       __syncthreads();
-      const int c = t >> 5, y = (t >> 3) & 3, z = t & 7;  // warp c sums component c of the plane's 32 nodes
+      const int c = nc, y = (t >> 3) & 3, z = t & 7;
 #pragma unroll
       for (int k = 0; k < MODAL_BLOCKS; ++k) {
         if (b0 + k >= nblocks) continue;
@@ -342,10 +357,10 @@ __global__ void __launch_bounds__(MODAL_THREADS, sizeof(T) == 8 ? 5 : 9) level0_
         T f = (ex[c][q] + ex[3 + c][qz]) + (ex[6 + c][q - 8] + ex[9 + c][z > 0 ? q - 9 : qz - 1]);
         const long node = long(b0 + k) * 128 + (x - 1) * 32 + (t & 31), g = node + c * N;
         if (OP == OP_RES) {
-          f = b[g] - f;
+          f = extra[k] - f;
         } else if (OP == OP_KUP) {
-          if (flags[node] & (DIR_X << c)) f = 0;
-          dot += double(u[g]) * double(f);
+          if (fl[k] & (DIR_X << c)) f = 0;
+          dot += double(extra[k]) * double(f);
         }
         out[g] = f;
       }
