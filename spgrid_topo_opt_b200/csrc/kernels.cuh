@@ -840,11 +840,18 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 8 : 5) stencil_op_kernel
   const int nbk = lane < 27 ? nbr[long(bi) * 27 + (X < 0 ? 0 : (X > 3 ? 2 : 1)) * 9 + (Y < 0 ? 0 : (Y > 3 ? 2 : 1)) * 3 +
                                   (Z < 0 ? 0 : (Z > 7 ? 2 : 1))]
                             : -1;
-  // an inactive node's row is all +0 (the operator build writes only the rows of
-  // active nodes into zeroed storage): its zeros come from registers, and its
-  // products with the neighbours' u are formed as before
+  // an inactive node's row is zero (the operator build writes only the rows of
+  // active nodes into zeroed storage): its result needs no neighbour
+  if (OP != SOP_GS && !(fl & ACTIVE_NODE)) {
+    pdl_wait();
+    if (lane < 3) {
+      const T r = OP == SOP_RES ? b[gidx + lane * N] : T(0);
+      out[gidx + lane * N] = (fl & (DIR_X << lane)) ? T(0) : (round_out ? T(round_to_float(r)) : r);
+    }
+    return;
+  }
   T a[9];
-  if (lane < 27 && (OP == SOP_GS || (fl & ACTIVE_NODE))) {
+  if (lane < 27) {
     const T* ap = A + gidx * 243 + lane * 9;
 #pragma unroll
     for (int k = 0; k < 9; ++k) a[k] = ap[k];
@@ -941,7 +948,8 @@ __global__ void __launch_bounds__(128) restrict_kernel(int nb, const int* __rest
   }
   pdl_wait();
   __syncthreads();
-  for (int h = e; h < RN; h += 128) {
+#pragma unroll 4
+  for (int h = e; h < RN; h += 128) {  // (four nodes of a thread in flight: the loop is bound by their latency)
     const int fx = x0 + h / (RY * RZ), fy = y0 + (h / RZ) % RY, fz = z0 + h % RZ;
     const int b = sblk[((fx >> 2) - bx0) * 9 + ((fy >> 2) - by0) * 3 + ((fz >> 3) - bz0)];
     T a = 0, c = 0, d = 0;
