@@ -14,6 +14,7 @@
 #include <algorithm>
 #include <array>
 #include <climits>
+#include <unordered_map>
 #include <vector>
 
 namespace sgs {
@@ -118,12 +119,25 @@ struct BottomOrder {
         lo[a] = l - 1;
         dim[a] = h - l + 3;
       }
-      std::vector<int> grid(size_t(dim[0]) * dim[1] * dim[2], -1);
-      auto cell = [&](int x, int y, int z) { return (size_t(x - lo[0]) * dim[1] + size_t(y - lo[1])) * dim[2] + size_t(z - lo[2]); };
-      for (size_t i = 0; i < at.size(); ++i) grid[cell(at[i][0], at[i][1], at[i][2])] = int(i);
+      // node at a place: a dense grid, or a map where the nodes are few and far apart
+      auto cell = [&](int x, int y, int z) { return (long(x - lo[0]) * dim[1] + (y - lo[1])) * dim[2] + (z - lo[2]); };
+      const long volume = long(dim[0]) * dim[1] * dim[2];
+      const bool dense = volume <= (1L << 24);
+      std::vector<int> grid(dense ? size_t(volume) : 0, -1);
+      std::unordered_map<long, int> sparse;
+      for (size_t i = 0; i < at.size(); ++i) {
+        const long c = cell(at[i][0], at[i][1], at[i][2]);
+        if (dense) grid[size_t(c)] = int(i);
+        else sparse.emplace(c, int(i));
+      }
+      auto node = [&](long c) {
+        if (dense) return grid[size_t(c)];
+        const auto it = sparse.find(c);
+        return it == sparse.end() ? -1 : it->second;
+      };
       for (size_t i = 0; i < at.size(); ++i)
         for (int q = 0; q < 27; ++q) {
-          const int j = grid[cell(at[i][0] + q / 9 - 1, at[i][1] + q / 3 % 3 - 1, at[i][2] + q % 3 - 1)];
+          const int j = node(cell(at[i][0] + q / 9 - 1, at[i][1] + q / 3 % 3 - 1, at[i][2] + q % 3 - 1));
           if (j < 0) continue;
           for (int r : {pos[i] / tile, (pos[i] + 2) / tile})
             for (int c : {pos[size_t(j)] / tile, (pos[size_t(j)] + 2) / tile}) on[size_t(r)][size_t(c)] = 1;
