@@ -35,7 +35,10 @@ struct BottomOrder {
     std::vector<int> tiles, first, ranges;
   };
   Phase phase[3];
-  bool single = true;                      // one leaf: phase 0 alone, with the full inverse
+  // no separators: phase 0 alone, with the full inverse.  (Not "one leaf": where
+  // the plane at one end holds more nodes than the rest, a cut through it leaves
+  // one leaf and that separator.)
+  bool single = true;
 
   void build(int tile_size) {
     tile = tile_size;
@@ -44,16 +47,14 @@ struct BottomOrder {
     ld = 0;
     std::vector<int> all(at.size());
     for (size_t i = 0; i < all.size(); ++i) all[i] = int(i);
-    leaf_of.clear();
-    leaves = 0;
+    leaf.clear();
     dissect(all);
-    single = leaves <= 1;
     symbolic();
+    single = phase[1].tiles.empty();
   }
 
  private:
-  std::vector<int> leaf_of;                // tile -> leaf, -1 for a separator's tiles
-  int leaves = 0;
+  std::vector<char> leaf;                  // tile -> whether it is a leaf's (else a separator's)
   // the axis of the largest extent of `nodes` and its range
   int longest(const std::vector<int>& nodes, int* lo, int* hi) const {
     int best = 0;
@@ -64,7 +65,7 @@ struct BottomOrder {
     }
     return best;
   }
-  void place(std::vector<int>& nodes, int axis, bool leaf) {
+  void place(std::vector<int>& nodes, int axis, bool is_leaf) {
     const int b = (axis + 1) % 3, c = (axis + 2) % 3;
     std::sort(nodes.begin(), nodes.end(), [&](int i, int j) {
       const auto &p = at[size_t(i)], &q = at[size_t(j)];
@@ -77,8 +78,7 @@ struct BottomOrder {
       ld += 3;
     }
     while (ld % tile) pad.push_back(int(ld++));
-    leaf_of.resize(size_t(ld / tile), leaf ? leaves : -1);
-    leaves += leaf;
+    leaf.resize(size_t(ld / tile), is_leaf);
   }
   void dissect(std::vector<int>& nodes) {
     if (nodes.empty()) return;
@@ -150,7 +150,7 @@ struct BottomOrder {
       int low = 0;
       std::vector<int> S;
       for (int J = 0; J < nt; ++J)
-        if (J != K && on[size_t(K)][size_t(J)] && (leaf_of[size_t(K)] >= 0 || leaf_of[size_t(J)] < 0)) {
+        if (J != K && on[size_t(K)][size_t(J)] && (leaf[size_t(K)] || !leaf[size_t(J)])) {
           S.push_back(J);
           low += J < K;
         }
@@ -165,11 +165,10 @@ struct BottomOrder {
       p = Phase();
       p.first.push_back(0);
       for (int I = 0; I < nt; ++I) {
-        const bool leaf = leaf_of[size_t(I)] >= 0;
-        if ((f == 1 && leaf) || (f == 2 && !leaf)) continue;
+        if ((f == 1 && leaf[size_t(I)]) || (f == 2 && !leaf[size_t(I)])) continue;
         p.tiles.push_back(I);
         for (int J = 0; J < nt; ++J) {
-          if (!on[size_t(I)][size_t(J)] || (leaf_of[size_t(J)] >= 0) != (f == 0)) continue;
+          if (!on[size_t(I)][size_t(J)] || bool(leaf[size_t(J)]) != (f == 0)) continue;
           if (int(p.ranges.size()) > 2 * p.first.back() && p.ranges.back() == J * tile) p.ranges.back() += tile;
           else p.ranges.insert(p.ranges.end(), {J * tile, (J + 1) * tile});
         }
