@@ -245,6 +245,11 @@ SGS_API int sgs_level_blocks(sgs_session* s, int level, int32_t* coords);
 SGS_API int sgs_level_flags(sgs_session* s, int level, uint32_t* flags);
 SGS_API int sgs_boundary_blocks(sgs_session* s, int level, int32_t* ordinals);
 
+/* The boundary-band groups of a level's smoothing: *slots the nodes a CTA of the
+ * cluster launch owns (0 where the band's colour passes are launched one by one,
+ * or there is none), *builds how often the level's band was examined for it. */
+SGS_API int sgs_band_group(sgs_session* s, int level, int32_t* slots, int32_t* builds);
+
 /* Apply one operator to host arrays in the compact layout [3][nblocks*128]:
  *  0 level-0 K*u            1 level-0 residual b - K u
  *  2 one smoothing sweep    (arg bit0 forward, bit1 boundary band only)

@@ -318,6 +318,7 @@ class Solver {
   std::vector<std::unique_ptr<Level<double>>> L64;
   std::vector<std::unique_ptr<Level<float>>> L32;
   std::vector<std::unique_ptr<BandTables>> band;  // per level; null where groups run pass by pass
+  std::vector<int> band_builds;                   // per level: how often band_tables looked at its band
   Bottom bottom;
   DevBuf<double> E64;
   DevBuf<float> E32;
@@ -628,15 +629,24 @@ class Solver {
     SGS_CUDA(cudaStreamSynchronize(stream));  // the temporaries go out of scope
   }
 
+  // dynamic shared memory a CTA of the boundary-band kernels may have
+  size_t band_smem_limit() {
+    int most = 0;
+    SGS_CUDA(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
+    return size_t(std::max(0, most - 1024));  // less the kernels' static shared memory
+  }
+  // what the plan takes of it on level l, in the V-cycle's precision
+  size_t band_smem_bytes(int l, const BandPlan& p) const {
+    return l > 0 ? (mixed() ? bandc_smem<float>(p) : bandc_smem<double>(p))
+                 : (mixed() ? band0_smem<float>(p) : band0_smem<double>(p));
+  }
   // Whether this device runs clusters of BG_CTAS CTAs of `kernel` with `smem`
   // bytes of shared memory each.
   template <typename K>
   bool cluster_runs(K kernel, size_t smem) {
-    int most = 0;
-    SGS_CUDA(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
-    most -= 1024;  // the kernels' static shared memory
-    if (smem > size_t(std::max(0, most))) return false;
-    bool ok = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most) == cudaSuccess &&
+    const size_t most = band_smem_limit();
+    if (smem > most) return false;
+    bool ok = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(most)) == cudaSuccess &&
               cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
     if (ok) {
       cudaLaunchConfig_t cfg = {};
@@ -658,10 +668,13 @@ class Solver {
 
   // Tables of level l's boundary-band groups from its node lists 8..15, if a
   // CTA's share of the band fits its shared memory in the V-cycle's precision.
-  // They depend on the hierarchy only: an operator update keeps them.
+  // They depend on the hierarchy only: an operator update keeps them, and a band
+  // that was refused is not looked at again.
   void band_tables(int l) {
     band.resize(P.levels.size());
-    if (band[l] || P.boundary_smoothing <= 0) return;
+    band_builds.resize(P.levels.size(), 0);
+    if (band_builds[l] || P.boundary_smoothing <= 0) return;
+    ++band_builds[l];
     Level<double>& d = *L64[l];
     if (d.nbound == 0) return;
     // the nodes a group updates, by colour (those that a level-0 pass only
@@ -689,7 +702,7 @@ class Solver {
       p.off[c] = p.slots;
       p.slots += most;
     }
-    if (p.slots > BG_SLOTS) return;
+    if (p.slots > BG_SLOTS || band_smem_bytes(l, p) > band_smem_limit()) return;  // (even without the halo)
     std::vector<int> table(size_t(BG_CTAS) * p.slots, BG_NONE);
     {
       int at[BG_CTAS][8] = {};
@@ -3654,6 +3667,14 @@ SGS_API int sgs_boundary_blocks(sgs_session* h, int level, int32_t* ordinals) {
   const HostLevel& L = h->solver->P.levels[level];
   if (ordinals) std::memcpy(ordinals, L.boundary.data(), L.boundary.size() * sizeof(int32_t));
   return int(L.boundary.size());
+}
+
+SGS_API int sgs_band_group(sgs_session* h, int level, int32_t* slots, int32_t* builds) {
+  if (!h || !slots || !builds || level < 0 || level >= h->solver->nlev()) return SGS_ERR_INPUT;
+  const Solver& S = *h->solver;
+  *slots = level < int(S.band.size()) && S.band[size_t(level)] ? S.band[size_t(level)]->plan.slots : 0;
+  *builds = level < int(S.band_builds.size()) ? S.band_builds[size_t(level)] : 0;
+  return 0;
 }
 
 SGS_API int sgs_apply(sgs_session* h, int op, int level, int arg, const double* in, const double* in2, double* out) {

@@ -29,7 +29,7 @@ EXPORTED_SYMBOLS = ("fem_solve", "fem_solve_free", "sgs_create", "sgs_destroy", 
                     "sgs_band_maps", "sgs_band_attach", "sgs_band_session", "sgs_band_step", "sgs_render",
                     "sgs_band_render", "sgs_band_get_flags", "sgs_band_filter_voxels", "sgs_band_kill_below",
                     "sgs_band_threshold_density", "sgs_solution_size", "sgs_set_density_device",
-                    "sgs_solution_device", "sgs_compliance_device", "sgs_sensitivity_device")
+                    "sgs_solution_device", "sgs_compliance_device", "sgs_sensitivity_device", "sgs_band_group")
 
 CELL_INSIDE, CELL_FORCE, CELL_FIXED = 1, 2, 4   # SGS_CELL_* (driver TopOptFlags bits 0-2)
 
@@ -176,6 +176,7 @@ def load(build_if_missing: bool = False):
     L.sgs_level_blocks.argtypes = [P, C.c_int, P]
     L.sgs_level_flags.argtypes = [P, C.c_int, P]
     L.sgs_boundary_blocks.argtypes = [P, C.c_int, P]
+    L.sgs_band_group.argtypes = [P, C.c_int, C.POINTER(C.c_int32), C.POINTER(C.c_int32)]
     L.sgs_apply.argtypes = [P, C.c_int, C.c_int, C.c_int, P, P, P]
     L.sgs_level_stencils.argtypes = [P, C.c_int, P, P]
     L.sgs_codec_roundtrip.argtypes = [P, C.c_int, C.POINTER(C.c_void_p)]
@@ -509,6 +510,13 @@ class Session:
         out = np.zeros(n, np.int32)
         load().sgs_boundary_blocks(self.h, level, _ptr(out))
         return out
+
+    def band_group(self, level: int):
+        """(nodes a CTA of the level's boundary-band groups owns, 0 where they run
+        pass by pass; how often the band was examined)."""
+        slots, builds = C.c_int32(0), C.c_int32(0)
+        self._check(load().sgs_band_group(self.h, level, C.byref(slots), C.byref(builds)))
+        return slots.value, builds.value
 
     def apply(self, op: int, level: int, x: np.ndarray, x2: Optional[np.ndarray] = None, arg: int = 0,
               out_level: Optional[int] = None) -> np.ndarray:

@@ -56,3 +56,18 @@ def test_reference_rounding_with_band_groups(native_lib, name):
     assert st["iterations"] == ref["iterations"]
     want = ref["displacements"][..., :3]
     assert np.abs(d[..., :3] - want).max() <= 1e-5 * np.abs(want).max()
+
+
+@pytest.mark.parametrize("precision", [native.PRECISION_FP64, native.PRECISION_MIXED])
+def test_refused_band_is_examined_once(native_lib, precision):
+    """The face of box80 is too large for a cluster on level 0, on level 2 (21^3
+    nodes) its stencil rows are too large for a cluster's shared memory in FP64:
+    density updates rebuild the operators and do not come back to it."""
+    inp = configs.to_inputs(configs.cantilever_box(80, density=(0.2, 1.0), bottom_size=10))
+    with native.Session(inp, precision=precision) as s:
+        assert s.levels == 4
+        for _ in range(2):
+            s.set_density(inp.density.data)
+        groups = [s.band_group(l) for l in range(s.levels)]
+    assert groups[0] == (0, 1)
+    assert (groups[2][0] > 0) == (precision == native.PRECISION_MIXED) and groups[2][1] == 1
