@@ -651,7 +651,7 @@ __global__ void __launch_bounds__(128, MINB) gs0_list4_kernel(const int* __restr
 }
 
 // The colour pass for few nodes (a boundary band, a small level: up to
-// GS_CELL_NODES): such a pass is bound by one thread's chain of dependent loads
+// GS_CELL_NODES of them): such a pass is bound by one thread's chain of dependent loads
 // and its 600 FMAs, so eight threads share a node, thread I taking the cell of
 // which the node is corner I.
 // The Q1 element is symmetric under reflections, K(I, J) = S K(0, I^J) S with S
@@ -662,9 +662,13 @@ __global__ void __launch_bounds__(128, MINB) gs0_list4_kernel(const int* __restr
 // eight threads with shuffles and thread 0 updates the node.  Same products as
 // gs0_list4_kernel, summed in another order.  PACKED: on u4 with nbrz, else on
 // the planes of u with E and nbr (-1 for missing blocks).
-// Both sides of GS_CELL_NODES: 614 nodes a pass (FP64, planes) 59 -> 26 us a sweep against a thread per
-// node, 1584 nodes 7.4 -> 4.7 us a pass; 15925 nodes (FP32) 33 against 44 us a sweep the other way.
-constexpr int GS_CELL_NODES = 6144;
+// The line is where a sweep takes as long either way (us a sweep of eight passes;
+// box with that many nodes a pass, eight threads / one thread a node):
+//   FP32 packed  14706 31.2 / 35.5, 20796 37.0 / 37.7, 32757 50.4 / 41.3
+//   FP64 packed   2460 29.7 / 34.2,  3048 30.4 / 28.6,  4492 32.0 / 28.6
+//   FP64 planes  34328 74.4 / 87.8, 44738 88.8 / 86.2, 57066 107.4 / 93.4
+template <typename T, bool PACKED>
+constexpr int GS_CELL_NODES = !PACKED ? 40960 : sizeof(T) == 4 ? 20480 : 2560;
 template <typename T, bool PACKED>
 __global__ void __launch_bounds__(128) gs0_cell_kernel(const int* __restrict__ list, int n,
                                                        const int* __restrict__ nbr,

@@ -1252,7 +1252,7 @@ class Solver {
         const int c = (boundary ? 8 : 0) + (forward ? k : 7 - k);
         const int lo = d.gs_off[c], cnt = d.gs_off[c + 1] - lo;
         if (cnt == 0) continue;
-        if (cnt <= GS_CELL_NODES) {  // few nodes: eight threads per node
+        if (cnt <= (u ? GS_CELL_NODES<T, false> : GS_CELL_NODES<T, true>)) {  // few nodes: eight threads per node
           if (!u)
             launch(gs0_cell_kernel<T, true>, blocks_for(long(cnt) * 8, 128), 128, 0, d.gs_list.p + lo, cnt, d.nbrz.p,
                    d.u4.p, nullptr, nullptr, b, d.flags.p, int(d.N), T(P.dx));
