@@ -16,21 +16,30 @@
 // subtracted from the right-hand side once, at the start.
 // Measured per V-cycle (three sweeps, four groups a level): 867 nodes in the
 // reference rounding 858 -> 292 us for the whole cycle (16^3 box), two levels of
-// 1260 and 645 nodes in FP32 629 -> 349 us (97 x 25 x 49 bridge), 7203 nodes in
-// FP64 559 -> 487 us (48^3 box).  A pass is bound by its chain: the cluster
-// barrier behind remote stores (about 800 cycles of an otherwise empty pass),
-// the shared loads, FMAs and shuffles.  With more nodes a CTA works through
-// several rounds a pass, and the separate launches, which spread over the whole
-// GPU, are faster (12354 nodes, 772 a CTA: 725 against 743 us): BG_SLOTS is the
-// line, and the tables of a CTA's share must fit its shared memory.
+// 1260 and 645 nodes in FP32 629 -> 349 us (97 x 25 x 49 bridge).  A pass is
+// bound by its chain: the cluster barrier behind remote stores (about 800 cycles
+// of an otherwise empty pass), the shared loads, FMAs and shuffles.  With more
+// nodes a CTA works through several rounds a pass, and the separate launches,
+// which spread over the whole GPU, are faster: band_slots() is the line, and the
+// tables of a CTA's share must fit its shared memory.
 #pragma once
 #include "kernels.cuh"
 
 namespace sgs {
 
-constexpr int BG_CTAS = 16, BG_THREADS = 512, BG_SLOTS = 640;
+constexpr int BG_CTAS = 16, BG_THREADS = 512;
 constexpr uint32_t BG_OUTSIDE = 0xffffffffu;
 constexpr int BG_NONE = INT32_MIN;  // unused slot
+
+// Slots a CTA (nodes it owns) up to which a level's groups run as one cluster.
+// V-cycles of boxes with the level's passes launched one by one / as a cluster (us):
+//   level 0, FP64           572 538 / 483,   620 542 / 506,   720 566 / 585
+//   level 0, ref. rounding  572 589 / 554,   620 585 / 574,   720 614 / 656
+//   level 0, FP32           515 370 / 355,   559 371 / 368,   608 392 / 407
+//   stencil level, FP32     140 658 / 623,   155 651 / 637,   176 713 / 727
+//   stencil level, FP64     101 749 / 735;   from about 105 on the rows do not fit
+template <typename T>
+constexpr int band_slots(int level) { return level > 0 ? 160 : sizeof(T) == 4 ? 560 : 640; }
 
 // The band's nodes in ascending order are cut into BG_CTAS equal parts (the
 // block order is a space-filling curve, so a part is compact); a CTA's nodes of

@@ -702,7 +702,8 @@ class Solver {
       p.off[c] = p.slots;
       p.slots += most;
     }
-    if (p.slots > BG_SLOTS || band_smem_bytes(l, p) > band_smem_limit()) return;  // (even without the halo)
+    if (p.slots > (mixed() ? band_slots<float>(l) : band_slots<double>(l))) return;
+    if (band_smem_bytes(l, p) > band_smem_limit()) return;  // (even without the halo)
     std::vector<int> table(size_t(BG_CTAS) * p.slots, BG_NONE);
     {
       int at[BG_CTAS][8] = {};

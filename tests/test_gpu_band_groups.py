@@ -71,3 +71,17 @@ def test_refused_band_is_examined_once(native_lib, precision):
         groups = [s.band_group(l) for l in range(s.levels)]
     assert groups[0] == (0, 1)
     assert (groups[2][0] > 0) == (precision == native.PRECISION_MIXED) and groups[2][1] == 1
+
+
+@pytest.mark.parametrize("n,precision,level,on", [
+    (48, native.PRECISION_MIXED, 0, True), (54, native.PRECISION_MIXED, 0, False),
+    (54, native.PRECISION_FP64, 0, True), (56, native.PRECISION_FP64, 0, False),
+    (82, native.PRECISION_MIXED, 2, True), (90, native.PRECISION_MIXED, 2, False),
+    (68, native.PRECISION_FP64, 2, True)])
+def test_lines_between_groups_and_passes(native_lib, n, precision, level, on):
+    """band_slots(): faces just below and above the size from which the passes are
+    faster launched one by one."""
+    inp = configs.to_inputs(configs.cantilever_box(n, density=(0.2, 1.0), bottom_size=12))
+    with native.Session(inp, precision=precision) as s:
+        assert s.levels > level + 1
+        assert (s.band_group(level)[0] > 0) == on
