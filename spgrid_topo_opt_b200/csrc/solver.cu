@@ -740,16 +740,17 @@ class Solver {
     SGS_CUDA(cudaStreamSynchronize(stream));
     for (int c : count) p.halo = std::max(p.halo, c);
     if (p.slots + p.halo >= BG_NOWHERE) return;
+    // the one kernel that this session's V-cycles launch on the level
     bool ok;
     if (l > 0)
       ok = mixed() ? cluster_runs(bandc_group_kernel<float>, bandc_smem<float>(p))
                    : cluster_runs(bandc_group_kernel<double>, bandc_smem<double>(p));
-    else if (mixed())  // the packed iterate of the V-cycle, the planes of the unit operators
-      ok = cluster_runs(band0_group_kernel<float, true>, band0_smem<float>(p)) &&
-           cluster_runs(band0_group_kernel<float, false>, band0_smem<float>(p));
+    else if (mixed())
+      ok = cluster_runs(band0_group_kernel<float, true>, band0_smem<float>(p));
+    else if (round_ref())
+      ok = cluster_runs(band0_group_kernel<double, false>, band0_smem<double>(p));
     else
-      ok = cluster_runs(band0_group_kernel<double, true>, band0_smem<double>(p)) &&
-           cluster_runs(band0_group_kernel<double, false>, band0_smem<double>(p));
+      ok = cluster_runs(band0_group_kernel<double, true>, band0_smem<double>(p));
     if (!ok) return;
     band[l] = std::move(t);
   }
@@ -768,9 +769,11 @@ class Solver {
     else if (!u)
       launch_group(band0_group_kernel<T, true>, band0_smem<T>(t.plan), t.plan, t.node.p, t.local.p, t.push.p,
                    t.hnode.p, t.hcount.p, d.nbr.p, d.u4.p, nullptr, Edev<T>(), b, d.flags.p, int(d.N), T(P.dx), count, int(forward), round);
-    else
+    else if constexpr (sizeof(T) == 8)
       launch_group(band0_group_kernel<T, false>, band0_smem<T>(t.plan), t.plan, t.node.p, t.local.p, t.push.p,
                    t.hnode.p, t.hcount.p, d.nbr.p, nullptr, u, Edev<T>(), b, d.flags.p, int(d.N), T(P.dx), count, int(forward), round);
+    else
+      throw CudaError("the FP32 V-cycle keeps level 0 packed", SGS_ERR_INTERNAL);
     ++launch_counter;
     return true;
   }
