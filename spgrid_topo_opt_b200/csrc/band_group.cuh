@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(BG_THREADS, 1) band0_group_kernel(
     BandPlan p, const int* __restrict__ node, const uint16_t* __restrict__ local, const uint16_t* __restrict__ push,
     const int* __restrict__ hnode, const int* __restrict__ hcount, const int* __restrict__ nbr, typename Pack4<T>::type* u4,
     T* u, const T* __restrict__ E, const T* __restrict__ b, const uint32_t* __restrict__ flags, int N, T dx,
-    int sweeps, int forward, int round) {
+    const KcReg<T> K, int sweeps, int forward, int round) {
   using V = typename Pack4<T>::type;
   extern __shared__ __align__(32) unsigned char band_mem[];
   const int S = p.slots;
@@ -195,8 +195,6 @@ __global__ void __launch_bounds__(BG_THREADS, 1) band0_group_kernel(
   constexpr int STEP = BG_THREADS / 8;
   const int Ix = I >> 2, Iy = (I >> 1) & 1, Iz = I & 1;
   const T s0 = Ix ? T(-1) : T(1), s1 = Iy ? T(-1) : T(1), s2 = Iz ? T(-1) : T(1);
-  KcReg<T> K;
-  K.load();
   const uint32_t to0 = cluster_address(su, 2 * I), to1 = cluster_address(su, 2 * I + 1);
   auto send = [&](uint32_t two, const V& v) {
     const uint32_t d0 = two & 0xffffu, d1 = two >> 16;

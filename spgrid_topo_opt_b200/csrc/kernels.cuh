@@ -14,16 +14,13 @@ namespace sgs {
 
 constexpr uint32_t ACTIVE_NODE = 0x10, DIR_X = 0x20, DIR_Y = 0x40, DIR_Z = 0x80, BOUNDARY_NODE = 0x1000;
 
-// Combined element matrix Kc[I][J][v][w] = mu0*K_mu + lambda0*K_la (set per solve)
-__constant__ double c_Kc64[8 * 8 * 9];
-__constant__ float c_Kc32[8 * 8 * 9];
-
+// Combined element matrix Kc[I][J][v][w] = mu0*K_mu + lambda0*K_la.  It and its
+// ten values below are launch arguments: sessions of several materials share the
+// device.
 template <typename T>
-__device__ __forceinline__ T kc(int idx);
-template <>
-__device__ __forceinline__ double kc<double>(int idx) { return c_Kc64[idx]; }
-template <>
-__device__ __forceinline__ float kc<float>(int idx) { return c_Kc32[idx]; }
+struct ElementMatrix {
+  T v[8 * 8 * 9];
+};
 
 __device__ __forceinline__ double round_to_float(double v) { return double(float(v)); }
 
@@ -32,7 +29,7 @@ __device__ __forceinline__ double round_to_float(double v) { return double(float
 // functions times 6 (mass {2, 1}, derivative-mass {-3, 3}, stiffness {6, -6});
 // the same formulas as element_tables() in solver.cu.  Up to sign the 576
 // entries take 10 values (m, l), so Kc = (mu0 m + lambda0 l) / 72 is 10 numbers,
-// which the single-precision level-0 kernels keep in registers (KcReg).
+// which the level-0 kernels keep in registers (KcReg).
 __host__ __device__ constexpr int q1_g(int a, int b, int i, int j) {
   int v = 1;
   for (int ax = 0; ax < 3; ++ax) {
@@ -53,16 +50,11 @@ __host__ __device__ constexpr int q1_class(int m, int l) {
        : (m == 10 && l == 4) ? 8 : (m == 32 && l == 8) ? 9 : -1;
 }
 constexpr int Q1_CLASS_M[10] = {3, 3, 4, 4, 6, 6, 8, 8, 10, 32}, Q1_CLASS_L[10] = {-3, 3, -2, 4, -6, 6, 2, 8, 4, 8};
-__constant__ float c_Kv32[10];   // (mu0 m_c + lambda0 l_c) / 72 per class, rounded like c_Kc32
-__constant__ double c_Kv64[10];  // the same in double, equal to the entries of c_Kc64
 
+// (mu0 m_c + lambda0 l_c) / 72 per class, in single precision rounded like the entries of Kc
 template <typename T>
 struct KcReg {
   T v[10];
-  __device__ __forceinline__ void load() {
-#pragma unroll
-    for (int c = 0; c < 10; ++c) v[c] = sizeof(T) == 4 ? T(c_Kv32[c]) : T(c_Kv64[c]);
-  }
   // Kc[I][J][r][s]; with constant arguments this folds to one register (and a sign)
   __device__ __forceinline__ T operator()(int I, int J, int r, int s) const {
     const int m = q1_mu72(I, J, r, s), l = q1_la72(I, J, r, s);
@@ -428,7 +420,8 @@ template <typename T, int MINB>
 __global__ void __launch_bounds__(128, MINB) gs0_list_kernel(const int* __restrict__ list, int n,
                                                              const int* __restrict__ nbr, const T* __restrict__ E,
                                                              T* u, const T* __restrict__ b,
-                                                             const uint32_t* __restrict__ flags, int N, T dx) {
+                                                             const uint32_t* __restrict__ flags, int N, T dx,
+                                                             const __grid_constant__ ElementMatrix<T> K) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) {
     pdl_wait();
@@ -487,18 +480,18 @@ __global__ void __launch_bounds__(128, MINB) gs0_list_kernel(const int* __restri
 #pragma unroll
         for (int v = 0; v < 3; ++v)
 #pragma unroll
-          for (int w = 0; w < 3; ++w) gc[I][v] = fma(kc<T>(k + v * 3 + w), up[p][w], gc[I][v]);
+          for (int w = 0; w < 3; ++w) gc[I][v] = fma(K.v[k + v * 3 + w], up[p][w], gc[I][v]);
       }
       if (Jx == 1) {  // last plane of this cell
 #pragma unroll
         for (int v = 0; v < 3; ++v) f[v] = fma(Ec[I], gc[I][v], f[v]);
         const int kd = (I * 8 + I) * 9;
-        dg[0] = fma(kc<T>(kd + 0), Ec[I], dg[0]);
-        dg[1] = fma(kc<T>(kd + 4), Ec[I], dg[1]);
-        dg[2] = fma(kc<T>(kd + 8), Ec[I], dg[2]);
-        dg[3] = fma(kc<T>(kd + 1), Ec[I], dg[3]);
-        dg[4] = fma(kc<T>(kd + 2), Ec[I], dg[4]);
-        dg[5] = fma(kc<T>(kd + 5), Ec[I], dg[5]);
+        dg[0] = fma(K.v[kd + 0], Ec[I], dg[0]);
+        dg[1] = fma(K.v[kd + 4], Ec[I], dg[1]);
+        dg[2] = fma(K.v[kd + 8], Ec[I], dg[2]);
+        dg[3] = fma(K.v[kd + 1], Ec[I], dg[3]);
+        dg[4] = fma(K.v[kd + 2], Ec[I], dg[4]);
+        dg[5] = fma(K.v[kd + 5], Ec[I], dg[5]);
       }
     }
   }
@@ -548,7 +541,8 @@ template <typename T, int MINB>
 __global__ void __launch_bounds__(128, MINB) gs0_list4_kernel(const int* __restrict__ list, int n,
                                                               const int* __restrict__ nbrz,
                                                               typename Pack4<T>::type* u4, const T* __restrict__ b,
-                                                              const uint32_t* __restrict__ flags, int N, T dx) {
+                                                              const uint32_t* __restrict__ flags, int N, T dx,
+                                                              const KcReg<T> K) {
   using V = typename Pack4<T>::type;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= n) {
@@ -573,8 +567,6 @@ __global__ void __launch_bounds__(128, MINB) gs0_list4_kernel(const int* __restr
   const int gy[3] = {packed_y((y + 3) & 3), packed_y(y), packed_y((y + 1) & 3)};
   const int gz[3] = {packed_z((z + 7) & 7), packed_z(z), packed_z((z + 1) & 7)};
   const int own = blk[0][0][0] + gx[1] + gy[1] + gz[1];
-  KcReg<T> K;
-  K.load();
   pdl_wait();
   if (raw < 0) {
     V v = u4[own];
@@ -674,7 +666,8 @@ __global__ void __launch_bounds__(128) gs0_cell_kernel(const int* __restrict__ l
                                                        const int* __restrict__ nbr,
                                                        typename Pack4<T>::type* u4, T* u, const T* __restrict__ E,
                                                        const T* __restrict__ b,
-                                                       const uint32_t* __restrict__ flags, int N, T dx) {
+                                                       const uint32_t* __restrict__ flags, int N, T dx,
+                                                       const KcReg<T> K) {
   using V = typename Pack4<T>::type;
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int k = t >> 3, I = t & 7;  // groups of 8 threads never straddle a warp
@@ -713,8 +706,6 @@ __global__ void __launch_bounds__(128) gs0_cell_kernel(const int* __restrict__ l
       if (Jp == I) at = idx[Jp];
     Ec = (raw < 0 || at < 0) ? T(0) : E[at];
   }
-  KcReg<T> K;
-  K.load();
   pdl_wait();
   if (raw < 0) {
     if (I == 0) {

@@ -18,7 +18,7 @@ namespace sgs {
 // ---------------------------------------------------------------------------
 
 // table[p][(a*8+b)*9 + v*3 + w], one thread per (p, a, b)
-__global__ void galerkin_table_kernel(int depth, double* __restrict__ table) {
+__global__ void galerkin_table_kernel(int depth, const __grid_constant__ ElementMatrix<double> K, double* __restrict__ table) {
   const long t = long(blockIdx.x) * blockDim.x + threadIdx.x;
   const int side = 1 << depth;
   const long npos = long(side) * side * side;
@@ -43,7 +43,7 @@ __global__ void galerkin_table_kernel(int depth, double* __restrict__ table) {
     for (int j = 0; j < 8; ++j) {
       const double w = Wa[i] * Wb[j];
       if (w == 0) continue;
-      for (int m = 0; m < 9; ++m) acc[m] += w * c_Kc64[(i * 8 + j) * 9 + m];
+      for (int m = 0; m < 9; ++m) acc[m] += w * K.v[(i * 8 + j) * 9 + m];
     }
   }
   double* out = table + p * 576 + (a * 8 + b) * 9;

@@ -459,7 +459,7 @@ class Solver {
       t0 = t;
     };
     const auto start = t0;
-    upload_constants();
+    element_constants();
     build_levels();
     mark(&setup_phase[0]);
     build_operators();
@@ -474,26 +474,37 @@ class Solver {
   double setup_phase[4] = {0, 0, 0, 0};
   double host_setup_seconds = 0;
 
-  void upload_constants() {
+  // the element matrix of this session's material (see ElementMatrix) and its ten values
+  ElementMatrix<double> kc_matrix;
+  ElementMatrix<float> kc_matrix32;
+  KcReg<double> kc64;
+  KcReg<float> kc32;
+  template <typename T>
+  const KcReg<T>& kc() const {
+    if constexpr (sizeof(T) == 4) return kc32;
+    else return kc64;
+  }
+  template <typename T>
+  const ElementMatrix<T>& kc_all() const {
+    if constexpr (sizeof(T) == 4) return kc_matrix32;
+    else return kc_matrix;
+  }
+  void element_constants() {
     double Kmu[8][8][3][3], Kla[8][8][3][3];
     element_tables(Kmu, Kla);
-    double kc64[576];
-    float kc32[576];
     for (int I = 0; I < 8; ++I)
       for (int J = 0; J < 8; ++J)
         for (int v = 0; v < 3; ++v)
           for (int w = 0; w < 3; ++w) {
-            double val = P.mu0 * Kmu[I][J][v][w] + P.lambda0 * Kla[I][J][v][w];
-            kc64[(I * 8 + J) * 9 + v * 3 + w] = val;
-            kc32[(I * 8 + J) * 9 + v * 3 + w] = float(val);
+            const int k = (I * 8 + J) * 9 + v * 3 + w;
+            kc_matrix.v[k] = P.mu0 * Kmu[I][J][v][w] + P.lambda0 * Kla[I][J][v][w];
+            kc_matrix32.v[k] = float(kc_matrix.v[k]);
           }
     // the 10 sign classes of the entries (q1_class); the integer formulas must
     // reproduce the element tables
-    float kv[10];
-    double kv64[10];
     for (int c = 0; c < 10; ++c) {
-      kv64[c] = P.mu0 * (double(Q1_CLASS_M[c]) / 72.0) + P.lambda0 * (double(Q1_CLASS_L[c]) / 72.0);
-      kv[c] = float(kv64[c]);
+      kc64.v[c] = P.mu0 * (double(Q1_CLASS_M[c]) / 72.0) + P.lambda0 * (double(Q1_CLASS_L[c]) / 72.0);
+      kc32.v[c] = float(kc64.v[c]);
     }
     for (int I = 0; I < 8; ++I)
       for (int J = 0; J < 8; ++J)
@@ -503,18 +514,13 @@ class Solver {
             const bool neg = m < 0 || (m == 0 && l < 0);
             const int c = q1_class(neg ? -m : m, neg ? -l : l);
             if (c < 0 || double(m) / 72.0 != Kmu[I][J][v][w] || double(l) / 72.0 != Kla[I][J][v][w] ||
-                (neg ? -kv[c] : kv[c]) != kc32[(I * 8 + J) * 9 + v * 3 + w] ||
-                (neg ? -kv64[c] : kv64[c]) != kc64[(I * 8 + J) * 9 + v * 3 + w])
+                (neg ? -kc64.v[c] : kc64.v[c]) != kc_matrix.v[(I * 8 + J) * 9 + v * 3 + w])
               throw CudaError("element table classes are inconsistent", SGS_ERR_INTERNAL);
             // the reflection symmetry gs0_cell_kernel relies on: K(I, J) = S K(0, I^J) S
             const double sg = ((I >> (2 - v)) & 1 ? -1.0 : 1.0) * ((I >> (2 - w)) & 1 ? -1.0 : 1.0);
             if (Kmu[I][J][v][w] != sg * Kmu[0][I ^ J][v][w] || Kla[I][J][v][w] != sg * Kla[0][I ^ J][v][w])
               throw CudaError("element table lacks the reflection symmetry", SGS_ERR_INTERNAL);
           }
-    SGS_CUDA(cudaMemcpyToSymbolAsync(c_Kv32, kv, sizeof(kv), 0, cudaMemcpyHostToDevice, stream));
-    SGS_CUDA(cudaMemcpyToSymbolAsync(c_Kv64, kv64, sizeof(kv64), 0, cudaMemcpyHostToDevice, stream));
-    SGS_CUDA(cudaMemcpyToSymbolAsync(c_Kc64, kc64, sizeof(kc64), 0, cudaMemcpyHostToDevice, stream));
-    SGS_CUDA(cudaMemcpyToSymbolAsync(c_Kc32, kc32, sizeof(kc32), 0, cudaMemcpyHostToDevice, stream));
   }
 
   template <typename T>
@@ -768,10 +774,10 @@ class Solver {
                    t.hcount.p, d.nbr.p, d.A.p, u, b, d.flags.p, d.N, count, int(forward), round);
     else if (!u)
       launch_group(band0_group_kernel<T, true>, band0_smem<T>(t.plan), t.plan, t.node.p, t.local.p, t.push.p,
-                   t.hnode.p, t.hcount.p, d.nbr.p, d.u4.p, nullptr, Edev<T>(), b, d.flags.p, int(d.N), T(P.dx), count, int(forward), round);
+                   t.hnode.p, t.hcount.p, d.nbr.p, d.u4.p, nullptr, Edev<T>(), b, d.flags.p, int(d.N), T(P.dx), kc<T>(), count, int(forward), round);
     else if constexpr (sizeof(T) == 8)
       launch_group(band0_group_kernel<T, false>, band0_smem<T>(t.plan), t.plan, t.node.p, t.local.p, t.push.p,
-                   t.hnode.p, t.hcount.p, d.nbr.p, nullptr, u, Edev<T>(), b, d.flags.p, int(d.N), T(P.dx), count, int(forward), round);
+                   t.hnode.p, t.hcount.p, d.nbr.p, nullptr, u, Edev<T>(), b, d.flags.p, int(d.N), T(P.dx), kc<T>(), count, int(forward), round);
     else
       throw CudaError("the FP32 V-cycle keeps level 0 packed", SGS_ERR_INTERNAL);
     ++launch_counter;
@@ -945,7 +951,7 @@ class Solver {
           DevBuf<double> table;
           DevBuf<int32_t> dorigin;
           table.alloc(size_t(npos) * 576);
-          galerkin_table_kernel<<<blocks_for(npos * 64, 128), 128, 0, stream>>>(lev, table.p);
+          galerkin_table_kernel<<<blocks_for(npos * 64, 128), 128, 0, stream>>>(lev, kc_matrix, table.p);
           dorigin.upload(origin, stream);
           const size_t smem = 2 * GT * 65 * sizeof(double);
           SGS_CUDA(cudaFuncSetAttribute(galerkin_cell_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
@@ -1259,10 +1265,10 @@ class Solver {
         if (cnt <= (u ? GS_CELL_NODES<T, false> : GS_CELL_NODES<T, true>)) {  // few nodes: eight threads per node
           if (!u)
             launch(gs0_cell_kernel<T, true>, blocks_for(long(cnt) * 8, 128), 128, 0, d.gs_list.p + lo, cnt, d.nbrz.p,
-                   d.u4.p, nullptr, nullptr, b, d.flags.p, int(d.N), T(P.dx));
+                   d.u4.p, nullptr, nullptr, b, d.flags.p, int(d.N), T(P.dx), kc<T>());
           else
             launch(gs0_cell_kernel<T, false>, blocks_for(long(cnt) * 8, 128), 128, 0, d.gs_list.p + lo, cnt, d.nbr.p,
-                   nullptr, u, Edev<T>(), b, d.flags.p, int(d.N), T(P.dx));
+                   nullptr, u, Edev<T>(), b, d.flags.p, int(d.N), T(P.dx), kc<T>());
           ++launch_counter;
           continue;
         }
@@ -1271,20 +1277,20 @@ class Solver {
           // despite a few spilled bytes); double: 128, 4 per SM
           if constexpr (sizeof(T) == 4)
             launch(gs0_list4_kernel<T, 8>, blocks_for(cnt, 128), 128, 0, d.gs_list.p + lo, cnt, d.nbrz.p, d.u4.p, b,
-                   d.flags.p, int(d.N), T(P.dx));
+                   d.flags.p, int(d.N), T(P.dx), kc<T>());
           else
             launch(gs0_list4_kernel<T, 4>, blocks_for(cnt, 128), 128, 0, d.gs_list.p + lo, cnt, d.nbrz.p, d.u4.p, b,
-                   d.flags.p, int(d.N), T(P.dx));
+                   d.flags.p, int(d.N), T(P.dx), kc<T>());
           ++launch_counter;
           continue;
         }
         // single precision: 80 registers, 6 CTAs per SM; double: 128, 4 per SM
         if constexpr (sizeof(T) == 4)
           launch(gs0_list_kernel<T, 6>, blocks_for(cnt, 128), 128, 0, d.gs_list.p + lo, cnt, d.nbr.p, Edev<T>(), u, b,
-                 d.flags.p, int(d.N), T(P.dx));
+                 d.flags.p, int(d.N), T(P.dx), kc_all<T>());
         else
           launch(gs0_list_kernel<T, 4>, blocks_for(cnt, 128), 128, 0, d.gs_list.p + lo, cnt, d.nbr.p, Edev<T>(), u, b,
-                 d.flags.p, int(d.N), T(P.dx));
+                 d.flags.p, int(d.N), T(P.dx), kc_all<T>());
         ++launch_counter;
       }
       return;
@@ -1996,7 +2002,7 @@ __global__ void pack_kernel(int nin, const int* __restrict__ in_block, const int
 // SIMP sensitivity per input-block cell (topo_opt/objective/minimal_compliance.cpp:86-146):
 // s_e = u_e^T (mu0 K_mu + lambda0 K_la) u_e (no dx), dc = p rho^(p-1) (1-Emin) s_e,
 // objective term s_e (Emin + rho^p (1-Emin)).
-__global__ void sensitivity_kernel(int nin, const int* __restrict__ in_block, const int* __restrict__ in_zoff,
+__global__ void sensitivity_kernel(const __grid_constant__ ElementMatrix<double> K, int nin, const int* __restrict__ in_block, const int* __restrict__ in_zoff,
                                    const int* __restrict__ nbr, const double* __restrict__ u, long N,
                                    const double* __restrict__ rho, double penalty, double emin, double* __restrict__ dc,
                                    double* __restrict__ se, double* __restrict__ obj_part) {
@@ -2020,7 +2026,7 @@ __global__ void sensitivity_kernel(int nin, const int* __restrict__ in_block, co
         for (int bb = 0; bb < 8; ++bb) {
           const int k = (a * 8 + bb) * 9;
           for (int i = 0; i < 3; ++i)
-            s += ue[a][i] * (c_Kc64[k + i * 3] * ue[bb][0] + c_Kc64[k + i * 3 + 1] * ue[bb][1] + c_Kc64[k + i * 3 + 2] * ue[bb][2]);
+            s += ue[a][i] * (K.v[k + i * 3] * ue[bb][0] + K.v[k + i * 3 + 1] * ue[bb][1] + K.v[k + i * 3 + 2] * ue[bb][2]);
         }
       dc[t] = s * pow(r, penalty - 1.0) * penalty * (1 - emin);
       objv = s * (emin + pow(r, penalty) * (1 - emin));
@@ -2043,7 +2049,7 @@ __global__ void sensitivity_kernel(int nin, const int* __restrict__ in_block, co
 // Gradient of the compliance per input-block cell for the PyTorch layer:
 // grad = factor * (*scale) * p rho^(p-1) (1-Emin) u_e^T K0 u_e (0 for empty cells),
 // u in the level-0 layout [3][N] (a saved solution).
-__global__ void sensitivity_grad_kernel(int nin, const int* __restrict__ in_block, const int* __restrict__ in_zoff,
+__global__ void sensitivity_grad_kernel(const __grid_constant__ ElementMatrix<double> K, int nin, const int* __restrict__ in_block, const int* __restrict__ in_zoff,
                                         const int* __restrict__ nbr, const double* __restrict__ u, long N,
                                         const double* __restrict__ rho, double penalty, double emin, double factor,
                                         const double* __restrict__ scale, double* __restrict__ grad) {
@@ -2070,7 +2076,7 @@ __global__ void sensitivity_grad_kernel(int nin, const int* __restrict__ in_bloc
     for (int bb = 0; bb < 8; ++bb) {
       const int k = (a * 8 + bb) * 9;
       for (int i = 0; i < 3; ++i)
-        s += ue[a][i] * (c_Kc64[k + i * 3] * ue[bb][0] + c_Kc64[k + i * 3 + 1] * ue[bb][1] + c_Kc64[k + i * 3 + 2] * ue[bb][2]);
+        s += ue[a][i] * (K.v[k + i * 3] * ue[bb][0] + K.v[k + i * 3 + 1] * ue[bb][1] + K.v[k + i * 3 + 2] * ue[bb][2]);
     }
   grad[t] = factor * (scale ? *scale : 1.0) * s * pow(r, penalty - 1.0) * penalty * (1 - emin);
 }
@@ -2653,7 +2659,7 @@ double Solver::sensitivity(const double* rho_host, double penalty, double emin, 
   se.alloc(size_t(nin) * 64);
   const unsigned nblk = blocks_for(nin * 64, 256);
   part.alloc(nblk);
-  sensitivity_kernel<<<nblk, 256, 0, stream>>>(int(nin), in_block.p, in_zoff.p, L64[0]->nbr.p, x.p, N0(), rho.p, penalty,
+  sensitivity_kernel<<<nblk, 256, 0, stream>>>(kc_matrix, int(nin), in_block.p, in_zoff.p, L64[0]->nbr.p, x.p, N0(), rho.p, penalty,
                                                emin, dc.p, se.p, part.p);
   std::vector<double> hp(nblk);
   SGS_CUDA(cudaMemcpyAsync(dc_host, dc.p, nin * 64 * sizeof(double), cudaMemcpyDeviceToHost, stream));
@@ -2801,7 +2807,7 @@ void Solver::design_step(const sgs_design_params& prm, sgs_design_result* out) {
   solve();
   const auto t1 = std::chrono::steady_clock::now();
   const unsigned nblk = blocks_for(nin * 64, 256);
-  sensitivity_kernel<<<nblk, 256, 0, stream>>>(int(nin), in_block.p, in_zoff.p, L64[0]->nbr.p, x.p, N0(),
+  sensitivity_kernel<<<nblk, 256, 0, stream>>>(kc_matrix, int(nin), in_block.p, in_zoff.p, L64[0]->nbr.p, x.p, N0(),
                                                design_rho.p, P.penalty, P.minimum_stiffness, design_dc.p,
                                                design_scratch.p, design_part.p);
   SGS_CUDA(cudaGetLastError());
@@ -2897,7 +2903,7 @@ void Solver::band_step(Band& B, const sgs_design_params& prm, sgs_design_result*
   const unsigned gs = blocks_for(ns, 256), gc = blocks_for(nc, 256);
   band_clear_kernel<<<gc, 256, 0, stream>>>(nc, B.fat.p, B.dc0.p);
   band_gather_kernel<<<gs, 256, 0, stream>>>(ns, B.sess_map.p, B.fat.p, B.flags.p, B.rho.p, design_scratch.p);
-  sensitivity_kernel<<<gs, 256, 0, stream>>>(int(nin), in_block.p, in_zoff.p, L64[0]->nbr.p, x.p, N0(),
+  sensitivity_kernel<<<gs, 256, 0, stream>>>(kc_matrix, int(nin), in_block.p, in_zoff.p, L64[0]->nbr.p, x.p, N0(),
                                              design_scratch.p, P.penalty, P.minimum_stiffness, design_dc.p,
                                              design_dc1.p, design_part.p);
   band_scatter_dc_kernel<<<gs, 256, 0, stream>>>(ns, B.sess_map.p, design_scratch.p, design_dc.p, B.dc0.p);
@@ -3528,7 +3534,7 @@ SGS_API int sgs_sensitivity_static(sgs_session* h, const double* density_dev, do
     if (nin == 0) {
       SGS_CUDA(cudaMemsetAsync(objective_dev, 0, sizeof(double), S.stream));
     } else {
-      sensitivity_kernel<<<unsigned(ncta), 256, 0, S.stream>>>(int(nin), S.in_block.p, S.in_zoff.p, S.L64[0]->nbr.p, S.x.p,
+      sensitivity_kernel<<<unsigned(ncta), 256, 0, S.stream>>>(S.kc_matrix, int(nin), S.in_block.p, S.in_zoff.p, S.L64[0]->nbr.p, S.x.p,
                                                               S.N0(), density_dev, S.P.penalty, S.P.minimum_stiffness,
                                                               dc_dev, element_energy_dev, part);
       sum_in_order_kernel<<<1, 32, 0, S.stream>>>(part, int(ncta), objective_dev);
@@ -3645,7 +3651,7 @@ SGS_API int sgs_sensitivity_device(sgs_session* h, const double* u_dev, const do
     const long nin = long(S.P.in_block.size());
     if (nin == 0) return;
     sensitivity_grad_kernel<<<blocks_for(nin * 64, 256), 256, 0, S.stream>>>(
-        int(nin), S.in_block.p, S.in_zoff.p, S.L64[0]->nbr.p, u_dev ? u_dev : S.x.p, S.N0(), density_dev,
+        S.kc_matrix, int(nin), S.in_block.p, S.in_zoff.p, S.L64[0]->nbr.p, u_dev ? u_dev : S.x.p, S.N0(), density_dev,
         S.P.penalty, S.P.minimum_stiffness, factor, scale_dev, grad_dev);
   });
 }
