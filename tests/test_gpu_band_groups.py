@@ -85,3 +85,13 @@ def test_lines_between_groups_and_passes(native_lib, n, precision, level, on):
     with native.Session(inp, precision=precision) as s:
         assert s.levels > level + 1
         assert (s.band_group(level)[0] > 0) == on
+
+
+@pytest.mark.parametrize("precision", [native.PRECISION_REFERENCE, native.PRECISION_FP64, native.PRECISION_MIXED])
+@pytest.mark.parametrize("name,on", [("box9", True), ("box33", True), ("shell40", True), ("bridge", True),
+                                     ("box72", False)])
+def test_which_inputs_run_level0_groups(native_lib, name, on, precision):
+    """The inputs above that are meant to test the cluster launches run them on
+    level 0, box72 the fallback."""
+    with native.Session(_inputs(name), precision=precision) as s:
+        assert (s.band_group(0)[0] > 0) == on

@@ -26,3 +26,30 @@ def test_bottom_solve_in_parts(native_lib, name):
         got, want = s.apply(native.OP_BOTTOM, top, b), o.apply(orc.OP_BOTTOM, top, b)
         assert s.solve(tolerance=1e-2)["bottom_unknowns"] > 4096
     assert np.abs(got - want).max() <= 1e-10 * np.abs(want).max()
+
+
+@pytest.mark.parametrize("precision,tol", [(native.PRECISION_FP64, 1e-9), (native.PRECISION_MIXED, 1e-4)])
+def test_bottom_in_parts_after_a_density_update(native_lib, precision, tol):
+    """New densities keep the order and its tables and fill the array again.  The
+    right-hand side is nonzero on unknowns only, so the bound is relative to the
+    solution: 1e-16 times the bottom's condition (stiffnesses of 0.008 to 1 over
+    15 nodes across: up to 1e6) in FP64; in mixed precision the V-cycle applies
+    an FP32 copy, whose rounding of 6e-8 grows by the cancellation in a row of
+    10^4 random terms, up to 10^2 in each of the three phases."""
+    prob = configs.cantilever_box(44, density=(0.2, 1.0), bottom_size=16)
+    rho = prob.density.copy()
+    prob.density = 1.2 - rho  # another design in the same range
+    new = configs.to_inputs(prob)
+    o = orc.Oracle(new, mode=orc.MODE_FP64)
+    prob.density = rho
+    with native.Session(configs.to_inputs(prob), precision=precision) as s:
+        top = s.levels - 1
+        fl, spokes = s.flags(top), s.stencils(top)[1]
+        free = np.stack([((spokes & 0x07FFFFFF) != 0) & ((fl & bit) == 0) for bit in (0x20, 0x40, 0x80)])
+        b = np.random.default_rng(4).standard_normal((3, len(fl))) * free
+        before = s.apply(native.OP_BOTTOM, top, b)
+        s.set_density(new.density.data)
+        got, want = s.apply(native.OP_BOTTOM, top, b), o.apply(orc.OP_BOTTOM, top, b)
+        assert s.solve(tolerance=1e-2)["bottom_unknowns"] > 4096
+    assert np.abs(got - want).max() <= tol * np.abs(want).max()
+    assert np.abs(before - want).max() > 0.01 * np.abs(want).max()
