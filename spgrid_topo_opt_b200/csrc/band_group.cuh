@@ -165,8 +165,10 @@ constexpr size_t bandc_smem(const BandPlan& p) { return band_smem<T>(p, 243 + 9)
 
 // Level 0, eight threads per node as in gs0_cell_kernel (thread I the cell of
 // which the node is corner I).  PACKED: the iterate is u4 (u, E), else the
-// planes of u.  What bounds a pass is its chain: 8 distributed loads, 24
-// dependent FMAs, three rounds of shuffles, the 3x3 update, the barrier.
+// planes of u.  What bounds a pass is its chain: 8 loads from the CTA's own
+// copies, 24 dependent FMAs, three rounds of shuffles, the 3x3 update, the remote
+// stores into the halos, the cluster barrier (16 SMs at 0.39 instructions a cycle
+// and scheduler, long-scoreboard and barrier stalls: 256^3 shell, FP32).
 template <typename T, bool PACKED>
 __global__ void __launch_bounds__(BG_THREADS, 1) band0_group_kernel(
     BandPlan p, const int* __restrict__ node, const uint16_t* __restrict__ local, const uint16_t* __restrict__ push,

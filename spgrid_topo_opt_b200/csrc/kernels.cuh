@@ -67,7 +67,8 @@ struct KcReg {
 // The level-0 operator at large sizes streams from HBM, whose latency its
 // resident warps do not cover: a CTA asks for the data of the one that will
 // follow it on the chip (about one wave of CTAs ahead) to be brought into L2
-// (1024^3 FP32 residual 1402 -> 1112 us).  The Gauss-Seidel passes, whose gathers
+// (1024^3, without it / with it: FP32 residual 1039 / 885 us, FP64 matvec 1824 /
+// 1801 us).  The Gauss-Seidel passes, whose gathers
 // keep more lines in flight, lost by it (1476 -> 1686 us a sweep), as by prefetches of their
 // later gathers into L1 (1453 -> 1574 us).
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
@@ -161,12 +162,16 @@ __device__ __forceinline__ void pdl_wait() {
 // 64 idle.  Cells without material (E = 0) skip the modal part.
 // PACKED: the iterate is the record u4 = (u, E) with the neighbour table nbrz
 // (a zero pad block for missing blocks), else the planes of u, E and nbr (-1).
-// Bound by latency: a CTA's five steps are a chain of loads, about 15 dependent
-// operations and a barrier each, and registers allow 5 CTAs an SM in FP64, 9 in
-// FP32 (4 / 8: 12% slower in FP64; 6 / 10, with spills: 23%).  At 1024^3 (340713
-// blocks), nodal form -> this: FP64 matvec 2240 -> 1830 us, FP32 residual 1348 ->
-// 890 us; 48^3 14.3 -> 8.3 us and 11.9 -> 8.6 us.  (The operands of the node phase
-// are requested at the step's start: 2010 and 962 us when loaded where used.)
+// Bound by L1 and by latency: the LSU data pipe is 81% busy in the FP32 residual,
+// 72% in FP64, 64% in the FP64 matvec (256^3 shell), and the stalls are the
+// plane loads (long scoreboard): a CTA's five steps are a chain of loads, about
+// 15 dependent operations and a barrier each.  Registers allow 5 CTAs an SM in
+// FP64, 9 in FP32, with 64 to 120 and 40 to 84 bytes spilled (1024^3 matvec and
+// residual 1801 and 885 us; 4 / 8 CTAs, without spills in FP64: 1786 and 867; 6 / 10,
+// 412 to 588 and 120 to 156 bytes: 2413 and 963).  At 1024^3 (340713 blocks), nodal
+// form -> this: FP64 matvec 2240 -> 1801 us, FP32 residual 1348 -> 885 us; 48^3
+// 14.3 -> 8.3 us and 11.9 -> 8.6 us.  (The operands of the node phase are
+// requested at the step's start: 2010 and 962 us when loaded where used.)
 // ---------------------------------------------------------------------------
 enum { OP_KU = 0, OP_RES = 1, OP_KUP = 2 };
 
@@ -514,7 +519,7 @@ __global__ void __launch_bounds__(128, MINB) gs0_list_kernel(const int* __restri
 // ---------------------------------------------------------------------------
 // Packed level 0 of the V-cycle (mixed and FP64 modes).  The iterate of level 0
 // is one record per node, (u_x, u_y, u_z, E of the node's cell): the 27-point
-// gathers of the smoother and the halo staging of the residual then read a
+// gathers of the smoother and the plane loads of the residual then read a
 // node's displacement and its cell's stiffness scale in one access (16 B in
 // FP32, 32 B in FP64), the same bytes as three planes of u plus the E plane.
 // ---------------------------------------------------------------------------
@@ -532,11 +537,11 @@ __global__ void reset_u4_kernel(typename Pack4<T>::type* __restrict__ u4, const 
 // (index nb) for missing neighbours, so the gathers need no test.  A node's
 // neighbourhood lies in at most eight blocks (a block is even, so a node next to
 // a face has one face per axis): their indices are loaded once, and each gather
-// selects one by the axes it crosses a face on.  Bound by L1 wavefronts (lines
-// of the gathers) and, where the iterate exceeds L2, by the DRAM traffic of
-// streaming it once a colour.  FP64 at 512^3 893 -> 664 us a
-// sweep, 48^3 47 -> 34 us; FP32 as before (1024^3 1463 us: 5.6 GB of iterate a
-// sweep at 4.4 TB/s).
+// selects one by the axes it crosses a face on.  Bound by the latency of the
+// gathers: at 256^3 (FP32) the long-scoreboard stalls lead at 42% of the warps
+// resident, with the LSU data pipe 40% and DRAM 45% busy.  Every colour streams
+// the iterate once: at 1024^3 8 x 0.70 GB, about 6.9 GB of DRAM traffic in 1411 us
+// a sweep (FP32).  FP64 at 512^3 893 -> 664 us a sweep by the layout, 48^3 47 -> 34 us.
 template <typename T, int MINB>
 __global__ void __launch_bounds__(128, MINB) gs0_list4_kernel(const int* __restrict__ list, int n,
                                                               const int* __restrict__ nbrz,

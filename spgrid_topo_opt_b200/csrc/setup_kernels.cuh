@@ -280,12 +280,13 @@ __global__ void identity_pad_kernel(double* M, long ld, const int* __restrict__ 
 // then T = P^-1 R, lower tiles A_IJ -= C_I T_J, A_IK = -C_I P^-1 (I > K),
 // A_KJ = T_J (J < K), A_KK = P^-1.  After the last pivot the lower tiles hold
 // the lower half of M^-1 and are mirrored.  I and J run over the tiles that row
-// K has reached (BottomOrder): with the unknowns in nested-dissection order the
-// steps of the 14739-unknown bottom of a 64^3 box touch about a ninth of the
-// tile products of a full elimination.  FP64 GEMM tiles of 128 x 128.
-// Measured (assembly, inverse and copies): 14739 unknowns 170 -> 35 ms, 20064
-// 409 -> 60 ms, 4287 10 -> 5 ms.  Steps on few tiles are bound by the chain
-// gather, row product, cross update, pivot; the last separators by the DMMA pipe.
+// K has reached (BottomOrder): with the unknowns in nested-dissection order and
+// separators eliminated among themselves, the steps of the 14739-unknown bottom
+// of a 64^3 box take a thirtieth of the tile products of a full elimination.
+// FP64 GEMM tiles of 128 x 128.  Measured (assembly, inverse and copies): 14739
+// unknowns 170 -> 22 ms, 20064 409 -> 30 ms, 9006 45 -> 13 ms, 4287 10 -> 6 ms.
+// Bound by the chain of a step (gather 6 us, row product 30, cross update 30,
+// beside it the next pivot 62): its products run on 5 to 30 SMs.
 // ---------------------------------------------------------------------------
 constexpr int SGJ = 128, SGJ_K = 16;
 
@@ -554,7 +555,9 @@ __global__ void bottom_gather_kernel(const int* __restrict__ node_pos, const T* 
 // the mixed V-cycle applies).  Row r is entry out[r] of the level's field u (-1:
 // padding).  PHASE 0: y = M x over the leaves' columns (plus x on the separators);
 // SINGLE: straight to u.  PHASE 1: xs = M y on the separators.  PHASE 2: u = y +
-// M xs on the leaves.  Bound by HBM: every entry is read once per application.
+// M xs on the leaves.  Every entry is read once per application, and the loads are in
+// flight for most of it: bound by their latency (9006 unknowns, FP32 copy, from DRAM:
+// 41 + 10 + 11 us for the phases, DRAM 36% busy in the first).
 template <typename TM>
 struct MatrixVec;
 template <>

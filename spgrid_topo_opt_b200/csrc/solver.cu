@@ -1460,7 +1460,7 @@ class Solver {
   }
 
   // K u (OP_KU) or b - K u (OP_RES) on the packed level-0 iterate: the tensor-core
-  // kernel in single precision, the shared-memory CUDA-core kernel otherwise
+  // kernel where the session asks for it (FP32), level0_modal_kernel otherwise
   template <typename T, int OP>
   void level0_packed(const T* b, T* out) {
     Level<T>& d = lev<T>(0);
@@ -1761,7 +1761,7 @@ __global__ void precond_out4_kernel(const typename Pack4<T>::type* __restrict__ 
 // them, K u vanishes where no active cell touches a node, x starts at zero), so
 // only the flags are read for them and the sectors that hold no active node are
 // never fetched.  They are bound by HBM; what they move per iteration and active
-// node is 44 + 116 + 88 B (mixed) and 3 vectors less than as separate steps: z
+// node is 44 + 132 + 88 B (mixed) and 3 vectors less than as separate steps: z
 // stays in the packed iterate (never written out as a planar vector), x is
 // updated together with the search direction, which reads s anyway, and the
 // packed iterate is cleared for the next V-cycle by the kernel that reads it last.
