@@ -286,7 +286,8 @@ __global__ void identity_pad_kernel(double* M, long ld, const int* __restrict__ 
 // FP64 GEMM tiles of 128 x 128.  Measured (assembly, inverse and copies): 14739
 // unknowns 170 -> 22 ms, 20064 409 -> 30 ms, 9006 45 -> 13 ms, 4287 10 -> 6 ms.
 // Bound by the chain of a step (gather 6 us, row product 30, cross update 30,
-// beside it the next pivot 62): its products run on 5 to 30 SMs.
+// beside it the next pivot 62): its products run on few SMs (5 to 28 of the 148
+// in the steps captured at 9006 unknowns).
 // ---------------------------------------------------------------------------
 constexpr int SGJ = 128, SGJ_K = 16;
 
