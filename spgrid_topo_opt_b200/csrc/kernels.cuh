@@ -664,6 +664,7 @@ __global__ void __launch_bounds__(128, MINB) gs0_list4_kernel(const int* __restr
 //   FP32 packed  14706 31.2 / 35.5, 20796 37.0 / 37.7, 32757 50.4 / 41.3
 //   FP64 packed   2460 29.7 / 34.2,  3048 30.4 / 28.6,  4492 32.0 / 28.6
 //   FP64 planes  34328 74.4 / 87.8, 44738 88.8 / 86.2, 57066 107.4 / 93.4
+// (FP32 planes: the unit sweep of a mixed session only, with the line of FP64.)
 template <typename T, bool PACKED>
 constexpr int GS_CELL_NODES = !PACKED ? 40960 : sizeof(T) == 4 ? 20480 : 2560;
 template <typename T, bool PACKED>
